@@ -118,8 +118,11 @@ typedef enum p2z_update_kind {
 } p2z_update_kind;
 
 /* How the work is laid onto the GPU.
- *  AUTO        FLAT for uniform events, PERSISTENT when event_ntrks or a hit mask is given.
- *  FLAT        one launch over every track slot of every event.
+ *  AUTO        FLAT; with a caller's hit mask and enough slots to fill the GPU more than once, FLAT
+ *              with P2Z_FLAG_SORT_WINDOWS.
+ *  FLAT        one launch over every track slot of every event (P2Z_UPDATE_V2 without missing
+ *              layers and without P2Z_FLAG_ACCURATE_TRIG or REFERENCE_ROUNDING, on 16-byte
+ *              aligned arrays: two tracks per thread when the launch fills the GPU).
  *  PER_EVENT   one launch per event (the reference's launch-per-chunk form,
  *              src/propagate-toz-test_CUDA_v4.cu:970-986, taken down to one event per launch).
  *  PERSISTENT  one persistent launch (grid = resident CTAs) whose warps take
@@ -168,14 +171,15 @@ typedef enum p2z_layout {
                                        = 10 (src/propagate-toz-test_CUDA_v4.cu:40-41, :972-986); the
                                        default issues them in order on the run's stream */
 #define P2Z_FLAG_SORT_WINDOWS 0x80u /* masked runs, FLAT / PERSISTENT: process each window of 128
-                                       consecutive slots in order of the slots' hit counts (a 1-byte
-                                       permutation the run computes on the device), so a warp's 32
+                                       consecutive slots in order of the slots' hit counts (a stable
+                                       order that each warp finds for itself; one flat launch, with
+                                       PERSISTENT too), so a warp's 32
                                        tracks take similar numbers of steps.  Per-track results are
-                                       the same.  On the uneven benchmark sample lane utilisation
-                                       rises from 60% to 85% and the persistent pass is 13% faster;
-                                       a warp's loads then reach 4 batches, so on even work (every
-                                       mask alike) it only costs.  p2z_autotune measures both for
-                                       masked runs, and runs with schedule AUTO sort when that
+                                       the same.  On uneven samples lane utilisation
+                                       rises from 60% to 85% and the pass is 6-16% faster;
+                                       a warp's loads then reach 4 batches; on even work (every
+                                       mask alike) it costs 2.5%.  p2z_autotune measures both for
+                                       masked runs, and runs with schedule AUTO then sort when that
                                        measured faster.  Packing an event's tracks in order of hit
                                        count (p2z_pack_by_hits_device, or when the arrays are built)
                                        gains more (99%) */
@@ -206,12 +210,13 @@ typedef struct p2z_config {
                             this context for the same key, else the rule under p2z_schedule */
   int32_t block_threads; /* threads per CTA, a multiple of 32 in 32..256; 0 -> the value
                             p2z_autotune measured best on this context for the same update,
-                            flags, bsize, layout and masking, else 128 */
+                            flags, bsize, layout and masking, else 32 (FLAT, PER_EVENT) or 128;
+                            the two-tracks-per-thread form uses at most 128 */
   uint32_t flags;        /* P2Z_FLAG_*; any other bit is P2Z_BAD_ARG */
   int32_t layout;        /* p2z_layout of the track, hit and output arrays */
   /* Uneven form (optional, host memory): nevts track counts.  NULL -> uniform. */
   const int64_t *event_ntrks;
-  int32_t threads_per_track; /* 1, or 2 (P2Z_UPDATE_V2 without REFERENCE_ROUNDING; FLAT,
+  int32_t threads_per_track; /* 1 (a thread may hold two tracks, see P2Z_SCHED_FLAT), or 2 (P2Z_UPDATE_V2 without REFERENCE_ROUNDING; FLAT,
                             PER_EVENT and PERSISTENT schedules): lanes 2i and 2i+1 of a warp
                             hold the same track and split the propagation of its covariance,
                             with bit-identical results.  0 -> the value p2z_autotune measured
@@ -309,10 +314,10 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
  * d_trk_out must not alias d_trk_in.  Calls on one context whose work
  * overlaps on the GPU (different streams, as the reference's GPU build issues
  * its chunks) share the context's device scratch: with the FLAT schedule
- * (the rule for runs without masks) and the default flags they share only the
+ * (the rule) and the default flags they share only the
  * status word, whose bits the kernels only set, and may overlap; with the
- * PERSISTENT or STAGED schedule (work counter), P2Z_FLAG_SORT_WINDOWS (window
- * permutation), uneven events given without a mask (padding mask), stats or
+ * PERSISTENT or STAGED schedule (work counter), uneven events given without a
+ * mask (padding mask), stats or
  * P2Z_FLAG_CHECK_INPUTS (status reset) they must not: order those streams, or
  * use one context per stream.  Replaces GPUsequence/GPUsequenceR
  * (src/propagate-toz-test_CUDA_v4.cu:746-828). */

@@ -23,18 +23,15 @@
 #endif
 // P2Z_FLAG_PER_EVENT_STREAMS: streams the per-event launches are spread over.
 constexpr int kEventStreams = 10;
-// Masked runs with P2Z_FLAG_SORT_WINDOWS: slots per sorted window.
-// A warp's 32 tracks take as many steps as the longest of them; with hit
-// counts of 5-20 per track, 32 slots taken in stored order keep 60% of the
-// lane-steps busy; sorted by hit count, windows of 64, 128 and 256 slots keep
-// 74%, 85% and 92%.  A sorted warp's loads reach as many batches of 32 as the
-// window holds, which costs per step: measured on one B200 (2000-event
-// sample, persistent schedule) 1.725, 1.668 and 2.189 ms against 1.894 ms in
-// stored order, so the window is 128 slots.
-#ifndef P2Z_SORT_WINDOW
-#define P2Z_SORT_WINDOW 128
-#endif
-
+// Threads per CTA where neither the caller nor the autotuner says: flat launches
+// take CTAs of one warp, which leave their registers as soon as the warp is done
+// (one B200, us per pass with 32 / 128: 1000 x 9600 tracks 1646 / 1651, 500 masked
+// events 606 / 610, 60 with the FP64 island sorted 161 / 168).  The FP32 kinds on
+// sorted windows take the window's four warps as one CTA: they read the same
+// sectors of hits, which one SM's L1 then holds for all of them (500 masked
+// events, under the power cap that a longer load meets, 627 / 577).  The queue
+// kernels' warps fetch their next work themselves.
+constexpr int kFlatBlock = 32, kSortedBlock = p2z::kSortWindow, kQueueBlock = 128;
 namespace p2z {
 cudaError_t launch_step(int bsize, float *trk, const float *hits, int64_t nslots, int nlayer, int layer, int what,
                         float kfact, cudaStream_t st);
@@ -84,7 +81,6 @@ struct p2z_context {
   // counts); empty when it holds anything else (a caller's mask copied by p2z_run)
   std::vector<int64_t> mask_key;
   DevBuf aux;                               // scratch of the validation reduction
-  DevBuf perm;                              // sorted-window permutation (masked runs)
   bool has_graph = false;
   GraphKey gkey;
   cudaGraphExec_t gexec = nullptr;
@@ -151,7 +147,7 @@ struct Plan {
   int upd = 0;
   int sc = SC_FAST;
   int schedule = P2Z_SCHED_FLAT;
-  int block = 0;
+  int block = 0;             // 0: kFlatBlock or kQueueBlock, by the schedule
   int tpt = 1;               // threads per track
   uint32_t flags = 0;
   int64_t nbatches = 0;
@@ -160,6 +156,7 @@ struct Plan {
   bool soa = false;          // P2Z_LAYOUT_SOA
   std::vector<int64_t> ev_slot_begin;  // nevts + 1 entries
   const int64_t *event_ntrks = nullptr;  // uneven: the caller's tracks per event
+  const uint32_t *padding_mask = nullptr;  // uneven without a caller's mask: internal_mask's
 };
 
 p2z_status make_plan(p2z_context *ctx, const p2z_config *cfg, Plan &pl) {
@@ -196,7 +193,7 @@ p2z_status make_plan(p2z_context *ctx, const p2z_config *cfg, Plan &pl) {
     pl.upd = UPDK_V2_REF;
   }
   pl.sc = (cfg->flags & P2Z_FLAG_ACCURATE_TRIG) ? SC_ACCURATE : SC_FAST;
-  pl.block = cfg->block_threads ? cfg->block_threads : 128;
+  pl.block = cfg->block_threads;
   if (cfg->threads_per_track < 0 || cfg->threads_per_track > 2)
     return fail(ctx, P2Z_UNSUPPORTED, "threads_per_track %d not in {0, 1, 2}", cfg->threads_per_track);
   if (cfg->threads_per_track == 2 && pl.upd != UPDK_V2)
@@ -272,38 +269,6 @@ __global__ void k_count_updates(const uint32_t *mask, int64_t nslots, uint32_t a
 
 uint32_t all_layers(int nlayer) { return nlayer >= 32 ? 0xffffffffu : ((1u << nlayer) - 1u); }
 
-// One CTA per window of `win` slots of [s0, s1): a counting sort of the
-// window's slots by hit count, most hits first, written as the within-window
-// offset of the slot each rank processes (perm[window base + rank]).  Ranks
-// of equal hit count are assigned by shared-memory atomics, so which thread
-// processes which of them varies from run to run; every track's arithmetic
-// is independent of its thread, so the results do not.
-__global__ void __launch_bounds__(P2Z_SORT_WINDOW) k_sort_windows(const uint32_t *__restrict__ mask, uint8_t *perm,
-                                                                  int64_t s0, int64_t s1, int win, uint32_t all) {
-  __shared__ int hist[33];
-  __shared__ int start[33];
-  const int i = threadIdx.x;
-  const int64_t base = s0 + (int64_t)blockIdx.x * win;
-  const int n = (int)min((int64_t)win, s1 - base);
-  if (i < 33) hist[i] = 0;
-  __syncthreads();
-  int key = 0, pos = 0;
-  if (i < n) {
-    key = 32 - __popc(__ldg(mask + base + i) & all);  // 0 = all 32 layers present
-    pos = atomicAdd(&hist[key], 1);
-  }
-  __syncthreads();
-  if (i == 0) {
-    int acc = 0;
-    for (int k = 0; k < 33; ++k) {
-      start[k] = acc;
-      acc += hist[k];
-    }
-  }
-  __syncthreads();
-  if (i < n) perm[base + start[key] + pos] = (uint8_t)i;
-}
-
 // The streams and events P2Z_FLAG_PER_EVENT_STREAMS spreads per-event launches
 // over, created on first use.
 p2z_status event_streams(p2z_context *ctx) {
@@ -339,9 +304,12 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   spec.upd = pl.upd;
   spec.sc = pl.sc;
   spec.masked = base.mask != nullptr;
-  spec.block = pl.block;
+  const bool flat = schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PER_EVENT;
+  spec.block = pl.block ? pl.block : (flat ? kFlatBlock : kQueueBlock);
   spec.grid = 0;
   spec.tpt = pl.tpt;
+  spec.duo = -1;
+  const bool padded = base.mask != nullptr && base.mask == pl.padding_mask;
   // Launches of at most 4 warps per SM leave each scheduler about one warp, with
   // nothing to run while it waits for a layer's hits from DRAM: those launches
   // ask L2 for their batches' hit blocks first (AOSOA).
@@ -366,6 +334,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
       spec.args.slot_begin = a;
       spec.args.slot_end = b;
       spec.args.l2_prefetch = prefetch_for(b - a);
+      spec.duo = duo_mode(spec, padded, ctx->num_sms);
       P2Z_CUDA(ctx, dispatch(spec, spread ? ctx->ev_streams[k++ % kEventStreams] : st));
       ++*launches;
     }
@@ -382,23 +351,13 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   if (s1 <= s0) return P2Z_OK;
   spec.args.l2_prefetch = prefetch_for(s1 - s0);  // (the staged kernel stages its hits itself)
   // masked flat and persistent runs: process each window's slots in order of hit count
-  const bool sort = spec.masked && (pl.flags & P2Z_FLAG_SORT_WINDOWS) &&
+  const bool sort = spec.masked && !padded && (pl.flags & P2Z_FLAG_SORT_WINDOWS) &&
                     (schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PERSISTENT);
-  if (sort) {
-    p2z_status r = ensure(ctx, ctx->perm, (size_t)pl.nslots);
-    if (r != P2Z_OK) return r;
-    spec.args.perm = (const uint8_t *)ctx->perm.p;
-    spec.args.win = P2Z_SORT_WINDOW;
-  }
-  auto launch_sort = [&](cudaStream_t s) {
-    const int64_t nwin = (s1 - s0 + P2Z_SORT_WINDOW - 1) / P2Z_SORT_WINDOW;
-    k_sort_windows<<<(unsigned)nwin, P2Z_SORT_WINDOW, 0, s>>>(base.mask, (uint8_t *)ctx->perm.p, s0, s1,
-                                                               P2Z_SORT_WINDOW, all_layers(pl.nlayer));
-    return cudaGetLastError();
-  };
-  if (schedule == P2Z_SCHED_FLAT) {
-    if (sort) P2Z_CUDA(ctx, launch_sort(st));
+  spec.args.sort = sort ? 1 : 0;
+  if (sort && !pl.block) spec.block = pl.upd == UPDK_3X3_F64 || pl.upd == UPDK_F64 ? kFlatBlock : kSortedBlock;
+  if (schedule == P2Z_SCHED_FLAT || sort) {
     spec.kind = KIND_FLAT;
+    spec.duo = duo_mode(spec, padded, ctx->num_sms);
     P2Z_CUDA(ctx, dispatch(spec, st));
     ++*launches;
     return P2Z_OK;
@@ -418,7 +377,6 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   P2Z_CUDA(ctx, cudaStreamIsCapturing(st, &cap));
   const bool use_graph = !(pl.flags & P2Z_FLAG_NO_GRAPH) && cap == cudaStreamCaptureStatusNone;
   if (!use_graph) {
-    if (sort) P2Z_CUDA(ctx, launch_sort(st));
     P2Z_CUDA(ctx, cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
     P2Z_CUDA(ctx, dispatch(spec, st));
     ++*launches;
@@ -448,9 +406,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
     cudaGraph_t g = nullptr;
     cudaStream_t cs = ctx->stream;
     P2Z_CUDA(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e0 = sort ? launch_sort(cs) : cudaSuccess;
     cudaError_t e1 = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), cs);
-    if (e1 == cudaSuccess) e1 = e0;
     cudaError_t e2 = dispatch(spec, cs);
     cudaError_t e3 = cudaStreamEndCapture(cs, &g);
     if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
@@ -491,7 +447,10 @@ int resolve_schedule(p2z_context *ctx, Plan &pl, const p2z_config *cfg, bool mas
     }
   }
   if (pl.schedule != P2Z_SCHED_AUTO) return pl.schedule;
-  return masked ? P2Z_SCHED_PERSISTENT : P2Z_SCHED_FLAT;
+  // one flat launch; of large runs with a caller's mask the windows are sorted (see sorted_offset)
+  if (masked && pl.padding_mask == nullptr && ctx && pl.nslots >= ctx->num_sms * kSortMinSlotsPerSm)
+    pl.flags |= P2Z_FLAG_SORT_WINDOWS;
+  return P2Z_SCHED_FLAT;
 }
 
 // Hit words an update kind reads per present layer: the 2-D updates the first
@@ -731,7 +690,7 @@ p2z_status p2z_destroy(p2z_context *c) {
     if (c->copy[i]) cudaStreamSynchronize(c->copy[i]);
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->run_exec) cudaGraphExecDestroy(c->run_exec);
-  for (DevBuf *b : {&c->trk, &c->hits, &c->out, &c->mask, &c->valid, &c->aux, &c->perm})
+  for (DevBuf *b : {&c->trk, &c->hits, &c->out, &c->mask, &c->valid, &c->aux})
     if (b->p) cudaFree(b->p);
   if (c->d_status) cudaFree(c->d_status);
   if (c->h_status) cudaFreeHost(c->h_status);
@@ -766,6 +725,7 @@ p2z_status p2z_run_device(p2z_context *ctx, const p2z_config *cfg, const void *d
   if (!mask && pl.uneven) {
     r = internal_mask(ctx, pl, st, &mask);
     if (r != P2Z_OK) return r;
+    pl.padding_mask = mask;
   }
   RunArgs base;
   std::memset(&base, 0, sizeof base);
@@ -853,6 +813,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
   if (!user_mask && pl.uneven) {
     r = internal_mask(ctx, pl, s0, &d_mask);
     if (r != P2Z_OK) return r;
+    pl.padding_mask = d_mask;
     P2Z_CUDA(ctx, cudaEventRecord(ctx->join[0], s0));
     P2Z_CUDA(ctx, cudaStreamWaitEvent(s1, ctx->join[0], 0));
   }
@@ -967,8 +928,6 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
                      (!user_mask || page_locked(hit_mask));
   if (graph) {
     // what enqueue_pass would allocate or create on first use, before recording
-    if (d_mask && (pl.flags & P2Z_FLAG_SORT_WINDOWS) && (r = ensure(ctx, ctx->perm, (size_t)pl.nslots)) != P2Z_OK)
-      return r;
     if (per_event && (pl.flags & P2Z_FLAG_PER_EVENT_STREAMS) && (r = event_streams(ctx)) != P2Z_OK) return r;
     int32_t kbits;
     std::memcpy(&kbits, &pl.kfact, sizeof kbits);
@@ -977,8 +936,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
                                 (int64_t)(uintptr_t)trk_in, (int64_t)(uintptr_t)hits, (int64_t)(uintptr_t)hit_mask,
                                 (int64_t)(uintptr_t)trk_out, (int64_t)(uintptr_t)ctx->trk.p,
                                 (int64_t)(uintptr_t)ctx->hits.p, (int64_t)(uintptr_t)ctx->out.p,
-                                (int64_t)(uintptr_t)ctx->mask.p, (int64_t)(uintptr_t)ctx->perm.p,
-                                (int64_t)(uintptr_t)d_mask};
+                                (int64_t)(uintptr_t)ctx->mask.p, (int64_t)(uintptr_t)d_mask};
     key.insert(key.end(), pl.ev_slot_begin.begin(), pl.ev_slot_begin.end());
     if (!(ctx->run_exec && ctx->run_key == key)) {
       if (ctx->run_exec) cudaGraphExecDestroy(ctx->run_exec);
