@@ -491,9 +491,9 @@ p2z_status p2z_prepare_hits(p2z_ref_rng *g, const p2z_ahit *hit_seeds, int nseed
 
 /* p2z_prepare generated on the device into device buffers (AOSOA, bsize
  * batches): the same words as p2z_prepare, for callers whose tracks and hits
- * live on the GPU.  The reference's rand() stream is split into chunks whose
+ * live on the GPU.  The reference's rand() stream is split into CTAs whose
  * starting states are computed by jumping its additive generator ahead, the
- * polar method's accepted attempts are counted per chunk and prefix-summed,
+ * polar method's accepted attempts are counted per CTA and prefix-summed,
  * and every variate is written to its word in parallel.  The variate's log is
  * correctly rounded where p2z_prepare calls the C library's logf (which
  * differs in the last place for ~0.3% of variates; that changed no output
