@@ -156,6 +156,7 @@ struct Plan {
   bool soa = false;          // P2Z_LAYOUT_SOA
   std::vector<int64_t> ev_slot_begin;  // nevts + 1 entries
   const int64_t *event_ntrks = nullptr;  // uneven: the caller's tracks per event
+  bool early = false;        // flat launches may be set up while the stream's previous kernel runs
   const uint32_t *padding_mask = nullptr;  // uneven without a caller's mask: internal_mask's
 };
 
@@ -295,6 +296,7 @@ bool page_locked(const void *p) {
 // queue: the persistent work counter to use.
 p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, int64_t s0, int64_t s1,
                         int schedule, cudaStream_t st, unsigned long long *queue, int *launches) {
+  const bool flat = schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PER_EVENT;
   LaunchSpec spec;
   spec.args = base;
   spec.args.queue = queue;
@@ -304,11 +306,11 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   spec.upd = pl.upd;
   spec.sc = pl.sc;
   spec.masked = base.mask != nullptr;
-  const bool flat = schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PER_EVENT;
   spec.block = pl.block ? pl.block : (flat ? kFlatBlock : kQueueBlock);
   spec.grid = 0;
   spec.tpt = pl.tpt;
   spec.duo = -1;
+  spec.early = flat && pl.early;
   const bool padded = base.mask != nullptr && base.mask == pl.padding_mask;
   // Launches of at most 4 warps per SM leave each scheduler about one warp, with
   // nothing to run while it waits for a layer's hits from DRAM: those launches
@@ -721,6 +723,7 @@ p2z_status p2z_run_device(p2z_context *ctx, const p2z_config *cfg, const void *d
   if (d_trk_in == d_trk_out && pl.nslots > 0) return fail(ctx, P2Z_BAD_ARG, "d_trk_out must not alias d_trk_in");
   P2Z_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+  pl.early = true;
   const uint32_t *mask = d_hit_mask;
   if (!mask && pl.uneven) {
     r = internal_mask(ctx, pl, st, &mask);

@@ -200,6 +200,7 @@ void launch_group(p2z_server *s) {
   std::memset(&spec, 0, sizeof spec);
   spec.tpt = 1;
   spec.duo = -1;
+  spec.early = false;
   spec.args.trk = s->d_trk;
   spec.args.hits = s->d_hit;
   spec.args.out = s->d_out;
