@@ -256,10 +256,52 @@ __device__ __forceinline__ void sin_versine(float a, float *s, float *v) {
     *v = 2.f * sh * sh;
   }
 }
-// sin and cos rounded once from a double evaluation: the correctly rounded
-// float result except within ~1e-16 of a rounding midpoint.
-__device__ __forceinline__ float sinf_cr(float x) { return (float)sin((double)x); }
-__device__ __forceinline__ float cosf_cr(float x) { return (float)cos((double)x); }
+// sin and cos of a float, each rounded once from a double evaluation: the
+// correctly rounded float result except within ~1e-16 of a rounding midpoint.
+// One reduction serves both: x = k pi/2 + r with pi/2 in two doubles, then the
+// Taylor series of sin r and cos r, |r| <= pi/4 (the next terms, r^19/19! and
+// r^18/18!, are below 1e-18).  Without CUDA's separate double sin and cos (whose
+// branch for arguments that need a longer pi/2 the last line keeps) the
+// reference-rounding step takes REFINSTR.
+__device__ __forceinline__ void sincosf_cr(float x, float *sn, float *cs) {
+  const double xd = (double)x;
+  if (__builtin_expect(!(fabsf(x) <= 1e5f), 0)) {
+    double s, c;
+    sincos(xd, &s, &c);
+    *sn = (float)s;
+    *cs = (float)c;
+    return;
+  }
+  // k: the nearest integer, in the low word of the sum with 1.5 2^52
+  double k = fma(xd, 0.6366197723675814, 6755399441055744.0);
+  const int q = __double2loint(k);
+  k -= 6755399441055744.0;
+  double r = fma(k, -1.5707963267948966, xd);
+  r = fma(k, -6.123233995736766e-17, r);
+  const double z = r * r;
+  double s = 1.0 / 355687428096000.0, c = 1.0 / 20922789888000.0;
+  s = fma(s, z, -1.0 / 1307674368000.0);
+  c = fma(c, z, -1.0 / 87178291200.0);
+  s = fma(s, z, 1.0 / 6227020800.0);
+  c = fma(c, z, 1.0 / 479001600.0);
+  s = fma(s, z, -1.0 / 39916800.0);
+  c = fma(c, z, -1.0 / 3628800.0);
+  s = fma(s, z, 1.0 / 362880.0);
+  c = fma(c, z, 1.0 / 40320.0);
+  s = fma(s, z, -1.0 / 5040.0);
+  c = fma(c, z, -1.0 / 720.0);
+  s = fma(s, z, 1.0 / 120.0);
+  c = fma(c, z, 1.0 / 24.0);
+  s = fma(s, z, -1.0 / 6.0);
+  c = fma(c, z, -0.5);
+  const float fc = (float)fma(c, z, 1.0);
+  // (sin r has r's sign, at r = -0 too)
+  const float fs = __uint_as_float((__float_as_uint((float)fma(z * r, s, r)) & 0x7fffffffu) |
+                                   ((unsigned)__double2hiint(r) & 0x80000000u));
+  const unsigned us = __float_as_uint((q & 1) ? fc : fs), uc = __float_as_uint((q & 1) ? fs : fc);
+  *sn = __uint_as_float(us ^ ((unsigned)(q & 2) << 30));
+  *cs = __uint_as_float(uc ^ ((unsigned)((q + 1) & 2) << 30));
+}
 
 // The unit vector (c, s) = (cos t, sin t) rotated to t + d, given w = sin d
 // and v = 1 - cos d: cos(t+d) = c - (c*v + s*w), sin(t+d) = s - (s*v - c*w).
@@ -603,25 +645,23 @@ __device__ __forceinline__ Jac<double> jacobian_f64(const Helix<double> &h, doub
 __device__ __forceinline__ Helix<float> propagate_params_ref(Trk<float, float> &s, float zout, float k) {
   Helix<float> h;
   h.deltaZ = zout - s.z;
-  h.pt = 1. / s.ipt;
-  h.cosP = cosf_cr(s.phi);
-  h.sinP = sinf_cr(s.phi);
-  const float cosT = cosf_cr(s.theta);
-  h.sinT = sinf_cr(s.theta);
+  // (the reference's 1./ipt and 1.0/cosT round a double quotient of floats to
+  // float: the float quotient itself, since 53 >= 2*24 + 2 bits)
+  h.pt = __fdiv_rn(1.f, s.ipt);
+  sincosf_cr(s.phi, &h.sinP, &h.cosP);
+  float cosT;
+  sincosf_cr(s.theta, &h.sinT, &cosT);
   const float pxin = h.cosP * h.pt;
   const float pyin = h.sinP * h.pt;
-  h.icosT = 1.0 / cosT;
+  h.icosT = __fdiv_rn(1.f, cosT);
   h.icosTk = h.icosT / k;
   const float alpha = h.deltaZ * h.sinT * s.ipt * h.icosTk;
-  h.sina = sinf_cr(alpha);
-  h.cosa = cosf_cr(alpha);
+  sincosf_cr(alpha, &h.sina, &h.cosa);
   s.x = s.x + k * (pxin * h.sina - pyin * (1. - h.cosa));
   s.y = s.y + k * (pyin * h.sina + pxin * (1. - h.cosa));
   s.z = zout;
   s.phi = s.phi + alpha;
-  h.sCPs = sinf_cr(h.cosP * h.sina);
-  const float cC = cosf_cr(h.cosP * h.sina);
-  h.omcC = cC;  // FORM_REFERENCE keeps cos(cosP*sina) itself here
+  sincosf_cr(h.cosP * h.sina, &h.sCPs, &h.omcC);  // FORM_REFERENCE keeps cos(cosP*sina) itself in omcC
   h.omc = 0.f;
   return h;
 }
