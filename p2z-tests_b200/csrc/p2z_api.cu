@@ -15,12 +15,21 @@
 #include "p2z.h"
 #include "p2z_kernels.cuh"
 
-// p2z_run: the host<->device copies and the kernels are pipelined over at most
-// this many chunks (alternating between two streams).  Measured on one B200 for
-// the 1000-event sample: 8 chunks 108.4 ms, 16 107.8 ms, 32 108.1-108.5 ms.
-#ifndef P2Z_RUN_MAX_CHUNKS
-#define P2Z_RUN_MAX_CHUNKS 16
-#endif
+// p2z_run: the host->device copies and the passes are pipelined over chunks, each
+// a third of what is left but no less than 64 batches and 1/64 of the run: a copy
+// costs about 4 us beside its bytes, so chunks are few and large, and what the
+// last pass and its outputs add after the last byte has arrived is small.
+constexpr int64_t kRunMinBatches = 64, kRunMinShare = 64;
+// Up to this many input bytes a run on page-locked arrays takes no copies at all:
+// the pass's loads cross the link, many warps' at a time, and so do its stores.
+// That reaches 50 GB/s in where the copies reach 55, but has no chunk to fill before
+// the first track and none to drain after the last, and copies in and out that
+// meet slow each other by 20-40 us a piece.  One B200, wall us a call, copies (the
+// best of 4-16 chunks) / direct: 1024 tracks 64 / 49, 9600 189 / 157, 16 x 9600 (91 MB)
+// 1954 / 1879, 64 x 9600 (364 MB) 7230 / 7274.  Batches narrower than 32 slots write
+// less than 128 bytes at a time (bsize 8: 2295 / 3524).
+constexpr size_t kRunDirectBytes = size_t(256) << 20;
+constexpr int kRunMaxChunks = 16;  // ln(64)/ln(3/2) + 1 of them at most, and the rest taken whole
 // P2Z_FLAG_PER_EVENT_STREAMS: streams the per-event launches are spread over.
 constexpr int kEventStreams = 10;
 // Threads per CTA where neither the caller nor the autotuner says: flat launches
@@ -72,7 +81,6 @@ struct p2z_context {
   cudaStream_t stream = nullptr;
   cudaStream_t copy[2] = {nullptr, nullptr};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
-  cudaEvent_t join[2] = {nullptr, nullptr};
   unsigned int *d_status = nullptr;         // device status word
   unsigned int *h_status = nullptr;         // page-locked copy of it (p2z_run)
   unsigned long long *d_queue = nullptr;    // 2 persistent work counters (one per copy stream)
@@ -87,12 +95,8 @@ struct p2z_context {
   std::vector<Tuned> tuned;                 // p2z_autotune results
   cudaStream_t ev_streams[kEventStreams] = {};  // P2Z_FLAG_PER_EVENT_STREAMS (created on first use)
   cudaEvent_t ev_fork = nullptr, ev_join[kEventStreams] = {};
-  // p2z_run's copy/kernel pipeline recorded as a graph (page-locked host buffers),
-  // with what it was recorded for and what it enqueues
-  cudaGraphExec_t run_exec = nullptr;
-  std::vector<int64_t> run_key;
-  int run_launches = 0;
-  int64_t run_h2d = 0, run_d2h = 0;
+  // p2z_run: chunk c's inputs have arrived; its pass is done
+  cudaEvent_t arrived[kRunMaxChunks] = {}, passed[kRunMaxChunks] = {};
   std::string last_error;
 };
 
@@ -156,6 +160,7 @@ struct Plan {
   bool soa = false;          // P2Z_LAYOUT_SOA
   std::vector<int64_t> ev_slot_begin;  // nevts + 1 entries
   const int64_t *event_ntrks = nullptr;  // uneven: the caller's tracks per event
+  bool host = false;         // the arrays are page-locked host memory
   bool early = false;        // flat launches may be set up while the stream's previous kernel runs
   const uint32_t *padding_mask = nullptr;  // uneven without a caller's mask: internal_mask's
 };
@@ -282,14 +287,15 @@ p2z_status event_streams(p2z_context *ctx) {
   return P2Z_OK;
 }
 
-// True for page-locked host memory (cudaHostAlloc / cudaHostRegister).
-bool page_locked(const void *p) {
+// The device's address of page-locked host memory (cudaHostAlloc, or
+// cudaHostRegister where the device can reach it), else null.
+float *mapped_host(const void *p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return nullptr;
   }
-  return a.type == cudaMemoryTypeHost;
+  return a.type == cudaMemoryTypeHost ? (float *)a.devicePointer : nullptr;
 }
 
 // Enqueue the hot-path launches of one pass over slots [s0, s1) on st.
@@ -316,7 +322,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   // nothing to run while it waits for a layer's hits from DRAM: those launches
   // ask L2 for their batches' hit blocks first (AOSOA).
   const int64_t small_slots = (int64_t)ctx->num_sms * 4 * 32 / pl.tpt;
-  auto prefetch_for = [&](int64_t n) { return (!pl.soa && n <= small_slots) ? 1 : 0; };
+  auto prefetch_for = [&](int64_t n) { return (!pl.soa && !pl.host && n <= small_slots) ? 1 : 0; };
   if (pl.tpt != 1 && schedule == P2Z_SCHED_STAGED)
     return fail(ctx, P2Z_UNSUPPORTED, "the staged schedule has one thread per track");
   if (schedule == P2Z_SCHED_PER_EVENT) {
@@ -336,7 +342,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
       spec.args.slot_begin = a;
       spec.args.slot_end = b;
       spec.args.l2_prefetch = prefetch_for(b - a);
-      spec.duo = duo_mode(spec, padded, ctx->num_sms);
+      spec.duo = duo_mode(spec, padded, pl.host ? 0 : ctx->num_sms);
       P2Z_CUDA(ctx, dispatch(spec, spread ? ctx->ev_streams[k++ % kEventStreams] : st));
       ++*launches;
     }
@@ -359,7 +365,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   if (sort && !pl.block) spec.block = pl.upd == UPDK_3X3_F64 || pl.upd == UPDK_F64 ? kFlatBlock : kSortedBlock;
   if (schedule == P2Z_SCHED_FLAT || sort) {
     spec.kind = KIND_FLAT;
-    spec.duo = duo_mode(spec, padded, ctx->num_sms);
+    spec.duo = duo_mode(spec, padded, pl.host ? 0 : ctx->num_sms);
     P2Z_CUDA(ctx, dispatch(spec, st));
     ++*launches;
     return P2Z_OK;
@@ -669,7 +675,10 @@ p2z_status p2z_create(int device, p2z_context **out) {
   if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) return bail("stream", e);
   for (int i = 0; i < 2; ++i) {
     if ((e = cudaStreamCreateWithFlags(&c->copy[i], cudaStreamNonBlocking)) != cudaSuccess) return bail("stream", e);
-    if ((e = cudaEventCreateWithFlags(&c->join[i], cudaEventDisableTiming)) != cudaSuccess) return bail("event", e);
+  }
+  for (int i = 0; i < kRunMaxChunks; ++i) {
+    if ((e = cudaEventCreateWithFlags(&c->arrived[i], cudaEventDisableTiming)) != cudaSuccess) return bail("event", e);
+    if ((e = cudaEventCreateWithFlags(&c->passed[i], cudaEventDisableTiming)) != cudaSuccess) return bail("event", e);
   }
   if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess) return bail("event", e);
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return bail("event", e);
@@ -691,14 +700,17 @@ p2z_status p2z_destroy(p2z_context *c) {
   for (int i = 0; i < 2; ++i)
     if (c->copy[i]) cudaStreamSynchronize(c->copy[i]);
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
-  if (c->run_exec) cudaGraphExecDestroy(c->run_exec);
   for (DevBuf *b : {&c->trk, &c->hits, &c->out, &c->mask, &c->valid, &c->aux})
     if (b->p) cudaFree(b->p);
   if (c->d_status) cudaFree(c->d_status);
   if (c->h_status) cudaFreeHost(c->h_status);
   if (c->d_queue) cudaFree(c->d_queue);
-  for (cudaEvent_t ev : {c->ev0, c->ev1, c->ev2, c->ev3, c->join[0], c->join[1], c->ev_fork})
+  for (cudaEvent_t ev : {c->ev0, c->ev1, c->ev2, c->ev3, c->ev_fork})
     if (ev) cudaEventDestroy(ev);
+  for (int i = 0; i < kRunMaxChunks; ++i) {
+    if (c->arrived[i]) cudaEventDestroy(c->arrived[i]);
+    if (c->passed[i]) cudaEventDestroy(c->passed[i]);
+  }
   for (int i = 0; i < kEventStreams; ++i) {
     if (c->ev_streams[i]) {
       cudaStreamSynchronize(c->ev_streams[i]);
@@ -801,9 +813,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
   const size_t tb = p2z_sizeof_mptrk(pl.B), hb = p2z_sizeof_mphit(pl.B);
   const size_t trk_bytes = tb * (size_t)pl.nbatches;
   const size_t hit_bytes = hb * (size_t)pl.nbatches * pl.nlayer;
-  if ((r = ensure(ctx, ctx->trk, trk_bytes)) != P2Z_OK) return r;
-  if ((r = ensure(ctx, ctx->hits, hit_bytes)) != P2Z_OK) return r;
-  if ((r = ensure(ctx, ctx->out, trk_bytes)) != P2Z_OK) return r;
+  const bool check = (pl.flags & P2Z_FLAG_CHECK_INPUTS) != 0;
   const bool user_mask = hit_mask != nullptr;
   const uint32_t *d_mask = nullptr;
   if (user_mask) {
@@ -812,169 +822,118 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
     ctx->mask_key.clear();
     d_mask = (const uint32_t *)ctx->mask.p;
   }
-  cudaStream_t s0 = ctx->copy[0], s1 = ctx->copy[1];
+  // sc carries the host->device copies; sp the passes and the copies back
+  cudaStream_t sc = ctx->copy[0], sp = ctx->copy[1];
   if (!user_mask && pl.uneven) {
-    r = internal_mask(ctx, pl, s0, &d_mask);
+    r = internal_mask(ctx, pl, sp, &d_mask);
     if (r != P2Z_OK) return r;
     pl.padding_mask = d_mask;
-    P2Z_CUDA(ctx, cudaEventRecord(ctx->join[0], s0));
-    P2Z_CUDA(ctx, cudaStreamWaitEvent(s1, ctx->join[0], 0));
   }
-  RunArgs base;
-  std::memset(&base, 0, sizeof base);
-  base.trk = (const float *)ctx->trk.p;
-  base.hits = (const float *)ctx->hits.p;
-  base.out = (float *)ctx->out.p;
-  base.mask = d_mask;
-  base.nlayer = pl.nlayer;
-  base.kfact = pl.kfact;
-  base.status = ctx->d_status;
-  int schedule = resolve_schedule(ctx, pl, cfg, d_mask != nullptr);
+  const int schedule = resolve_schedule(ctx, pl, cfg, d_mask != nullptr);
   // The per-event form is timed as it stands: copies first, then one launch per event.
   const bool per_event = schedule == P2Z_SCHED_PER_EVENT;
   // Only the 2-D updates read just the first 6 of the 9 hit words.
   const bool six = (pl.upd == UPDK_V2 || pl.upd == UPDK_V2_COMP || pl.upd == UPDK_F64 || pl.upd == UPDK_V2_REF) &&
                    !(pl.flags & P2Z_FLAG_FULL_HITS);
-  const int64_t nchunk = per_event ? 1 : std::max<int64_t>(1, std::min<int64_t>(P2Z_RUN_MAX_CHUNKS, pl.nbatches / 64));
-  const int64_t cb = nchunk ? (pl.nbatches + nchunk - 1) / nchunk : 0;
+  const size_t read_bytes = trk_bytes + hit_bytes / 9 * (six ? 6 : 9);
+  // Page-locked arrays, every layer present: one pass reads and writes them over the
+  // link itself (see kRunDirectBytes).
+  const float *h_trk = nullptr, *h_hits = nullptr;
+  float *h_out = nullptr;
+  if (pl.nslots > 0 && !user_mask && !check && !per_event && !(pl.flags & P2Z_FLAG_FULL_HITS) &&
+      (pl.soa || pl.B >= 32) && read_bytes <= kRunDirectBytes) {
+    h_trk = mapped_host(trk_in);
+    h_hits = mapped_host(hits);
+    h_out = mapped_host(trk_out);
+  }
+  const bool direct = h_trk && h_hits && h_out;
+  if (!direct) {
+    if ((r = ensure(ctx, ctx->trk, trk_bytes)) != P2Z_OK) return r;
+    if ((r = ensure(ctx, ctx->hits, hit_bytes)) != P2Z_OK) return r;
+    if ((r = ensure(ctx, ctx->out, trk_bytes)) != P2Z_OK) return r;
+  }
+  pl.host = direct;
+  RunArgs base;
+  std::memset(&base, 0, sizeof base);
+  base.trk = direct ? h_trk : (const float *)ctx->trk.p;
+  base.hits = direct ? h_hits : (const float *)ctx->hits.p;
+  base.out = direct ? h_out : (float *)ctx->out.p;
+  base.mask = d_mask;
+  base.nlayer = pl.nlayer;
+  base.kfact = pl.kfact;
+  base.status = ctx->d_status;
+  std::vector<int64_t> first = {0};  // batches [first[c], first[c + 1])
+  while (first.back() < pl.nbatches) {
+    const int64_t left = pl.nbatches - first.back();
+    const int64_t least = std::max(kRunMinBatches, pl.nbatches / kRunMinShare);
+    const int64_t take = per_event || direct ? left : std::max(least, left / 3);
+    first.push_back(left - take < least || first.size() == kRunMaxChunks ? pl.nbatches : first.back() + take);
+  }
+  const int nchunk = (int)first.size() - 1;
   int launches = 0;
   int64_t h2d = 0, d2h = 0;
-  // P2Z_FLAG_CHECK_INPUTS: each chunk is scanned after its copies, before its pass
-  const bool check = (pl.flags & P2Z_FLAG_CHECK_INPUTS) != 0;
-  // The work of one call on the two copy streams: the status reset, then per
-  // chunk the host->device copies, the pass and the device->host copy,
-  // alternating between s0 and s1 (s1 forks from and joins back into s0).
-  auto pipeline = [&]() -> p2z_status {
-    P2Z_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned int), s0));
-    P2Z_CUDA(ctx, cudaEventRecord(ctx->join[0], s0));
-    P2Z_CUDA(ctx, cudaStreamWaitEvent(s1, ctx->join[0], 0));
-    for (int it = 0; it < pl.niter; ++it) {
-      for (int64_t c = 0; c < nchunk; ++c) {
-        cudaStream_t st = (c & 1) ? s1 : s0;
-        const int64_t b0 = c * cb, b1 = std::min(pl.nbatches, b0 + cb);
-        if (b1 <= b0) continue;
-        const int64_t nbc = b1 - b0;
-        if (pl.soa) {
-          // slots [b0*B, b1*B) of every element row: pitched copies
-          r = copy_soa_chunk(ctx, pl, trk_in, hits, b0 * pl.B, nbc * pl.B, six, st, &h2d);
-          if (r != P2Z_OK) return r;
-        } else {
-          P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->trk.p + b0 * tb, (const char *)trk_in + b0 * tb, nbc * tb,
-                                        cudaMemcpyHostToDevice, st));
-          h2d += nbc * tb;
-          const size_t hrow = hb, hrows = (size_t)nbc * pl.nlayer;
-          const size_t hoff = (size_t)b0 * pl.nlayer * hb;
-          if (six) {
-            const size_t w = 6 * (size_t)pl.B * 4;
-            P2Z_CUDA(ctx, cudaMemcpy2DAsync((char *)ctx->hits.p + hoff, hrow, (const char *)hits + hoff, hrow, w, hrows,
-                                            cudaMemcpyHostToDevice, st));
-            h2d += (int64_t)(w * hrows);
-          } else {
-            P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->hits.p + hoff, (const char *)hits + hoff, hrow * hrows,
-                                          cudaMemcpyHostToDevice, st));
-            h2d += (int64_t)(hrow * hrows);
-          }
-        }
-        if (user_mask) {
-          P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->mask.p + b0 * pl.B * 4, (const char *)hit_mask + b0 * pl.B * 4,
-                                        nbc * pl.B * 4, cudaMemcpyHostToDevice, st));
-          h2d += nbc * pl.B * 4;
-        }
-        if (check) {
-          r = enqueue_check(ctx, pl, base, b0 * pl.B, b1 * pl.B, st);
-          if (r != P2Z_OK) return r;
-        }
-        if (!per_event) {
-          r = enqueue_pass(ctx, pl, base, b0 * pl.B, b1 * pl.B,
-                           (schedule == P2Z_SCHED_PERSISTENT || schedule == P2Z_SCHED_STAGED) ? P2Z_SCHED_FLAT : schedule,
-                           st, ctx->d_queue + (c & 1), &launches);
-          if (r != P2Z_OK) return r;
-          if (pl.soa) {
-            const size_t pitch = (size_t)pl.nslots * 4, off = (size_t)b0 * pl.B * 4, w = (size_t)nbc * pl.B * 4;
-            P2Z_CUDA(ctx, cudaMemcpy2DAsync((char *)trk_out + off, pitch, (const char *)ctx->out.p + off, pitch, w,
-                                            TRK_WORDS, cudaMemcpyDeviceToHost, st));
-          } else {
-            P2Z_CUDA(ctx, cudaMemcpyAsync((char *)trk_out + b0 * tb, (const char *)ctx->out.p + b0 * tb, nbc * tb,
-                                          cudaMemcpyDeviceToHost, st));
-          }
-          d2h += nbc * tb;
-        }
-      }
-      if (per_event) {
-        r = enqueue_pass(ctx, pl, base, 0, pl.nslots, P2Z_SCHED_PER_EVENT, s0, ctx->d_queue, &launches);
+  P2Z_CUDA(ctx, cudaEventRecord(ctx->ev0, sc));
+  P2Z_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned int), sp));
+  // The copies in follow one another on a stream of their own, so that the link
+  // into the GPU is never idle between chunks; a chunk's pass waits for its
+  // copies only, and a chunk is copied over (niter > 1) once its pass is done.
+  for (int it = 0; it < pl.niter; ++it) {
+    for (int c = 0; c < nchunk; ++c) {
+      const int64_t b0 = first[c], b1 = first[c + 1], nbc = b1 - b0;
+      if (it > 0) P2Z_CUDA(ctx, cudaStreamWaitEvent(sc, ctx->passed[c], 0));
+      if (direct) {
+        h2d += (int64_t)read_bytes;
+      } else if (pl.soa) {
+        // slots [b0*B, b1*B) of every element row: pitched copies
+        r = copy_soa_chunk(ctx, pl, trk_in, hits, b0 * pl.B, nbc * pl.B, six, sc, &h2d);
         if (r != P2Z_OK) return r;
-        P2Z_CUDA(ctx, cudaMemcpyAsync(trk_out, ctx->out.p, trk_bytes, cudaMemcpyDeviceToHost, s0));
-        d2h += trk_bytes;
+      } else {
+        P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->trk.p + b0 * tb, (const char *)trk_in + b0 * tb, nbc * tb,
+                                      cudaMemcpyHostToDevice, sc));
+        h2d += nbc * tb;
+        const size_t hrow = hb, hrows = (size_t)nbc * pl.nlayer;
+        const size_t hoff = (size_t)b0 * pl.nlayer * hb;
+        if (six) {
+          const size_t w = 6 * (size_t)pl.B * 4;
+          P2Z_CUDA(ctx, cudaMemcpy2DAsync((char *)ctx->hits.p + hoff, hrow, (const char *)hits + hoff, hrow, w, hrows,
+                                          cudaMemcpyHostToDevice, sc));
+          h2d += (int64_t)(w * hrows);
+        } else {
+          P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->hits.p + hoff, (const char *)hits + hoff, hrow * hrows,
+                                        cudaMemcpyHostToDevice, sc));
+          h2d += (int64_t)(hrow * hrows);
+        }
       }
+      if (user_mask) {
+        P2Z_CUDA(ctx, cudaMemcpyAsync((char *)ctx->mask.p + b0 * pl.B * 4, (const char *)hit_mask + b0 * pl.B * 4,
+                                      nbc * pl.B * 4, cudaMemcpyHostToDevice, sc));
+        h2d += nbc * pl.B * 4;
+      }
+      P2Z_CUDA(ctx, cudaEventRecord(ctx->arrived[c], sc));
+      P2Z_CUDA(ctx, cudaStreamWaitEvent(sp, ctx->arrived[c], 0));
+      if (check) {
+        r = enqueue_check(ctx, pl, base, b0 * pl.B, b1 * pl.B, sp);
+        if (r != P2Z_OK) return r;
+      }
+      r = enqueue_pass(ctx, pl, base, b0 * pl.B, b1 * pl.B,
+                       (schedule == P2Z_SCHED_PERSISTENT || schedule == P2Z_SCHED_STAGED) ? P2Z_SCHED_FLAT : schedule,
+                       sp, ctx->d_queue, &launches);
+      if (r != P2Z_OK) return r;
+      if (direct) {
+      } else if (pl.soa && !per_event) {
+        const size_t pitch = (size_t)pl.nslots * 4, off = (size_t)b0 * pl.B * 4, w = (size_t)nbc * pl.B * 4;
+        P2Z_CUDA(ctx, cudaMemcpy2DAsync((char *)trk_out + off, pitch, (const char *)ctx->out.p + off, pitch, w,
+                                        TRK_WORDS, cudaMemcpyDeviceToHost, sp));
+      } else {
+        P2Z_CUDA(ctx, cudaMemcpyAsync((char *)trk_out + b0 * tb, (const char *)ctx->out.p + b0 * tb, nbc * tb,
+                                      cudaMemcpyDeviceToHost, sp));
+      }
+      d2h += nbc * tb;
+      if (it + 1 < pl.niter) P2Z_CUDA(ctx, cudaEventRecord(ctx->passed[c], sp));
     }
-    P2Z_CUDA(ctx, cudaEventRecord(ctx->join[1], s1));
-    P2Z_CUDA(ctx, cudaStreamWaitEvent(s0, ctx->join[1], 0));
-    P2Z_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, s0));
-    return P2Z_OK;
-  };
-  // With page-locked host buffers a pipeline of at least kRunGraphMinChunks
-  // passes over chunks (or per-event launches; niter passes each) is recorded once as a CUDA graph and
-  // replayed while the plan and every buffer it touches stay the same: a call
-  // then costs one graph launch instead of enqueueing each copy and kernel (up
-  // to 16 chunks x 4-5 operations, or one launch per event).  A shorter
-  // pipeline is enqueued directly: its first copy then starts while the rest
-  // is still being enqueued, which a graph launch does not allow (one B200,
-  // one event from page-locked buffers: direct 3-6 us faster per call from
-  // 256 to 4096 tracks, one and two chunks; the graph 1 us faster at 9600
-  // tracks, four chunks).  Pageable buffers are copied through the driver's
-  // staging path, which a graph cannot hold, so they take the direct path, as
-  // does P2Z_FLAG_NO_GRAPH.
-  constexpr int64_t kRunGraphMinChunks = 4;
-  const int64_t pipeline_ops = (per_event ? (int64_t)pl.ev_slot_begin.size() - 1 : nchunk) * pl.niter;
-  const bool graph = !(pl.flags & P2Z_FLAG_NO_GRAPH) && pl.nslots > 0 && pipeline_ops >= kRunGraphMinChunks &&
-                     page_locked(trk_in) && page_locked(hits) && page_locked(trk_out) &&
-                     (!user_mask || page_locked(hit_mask));
-  if (graph) {
-    // what enqueue_pass would allocate or create on first use, before recording
-    if (per_event && (pl.flags & P2Z_FLAG_PER_EVENT_STREAMS) && (r = event_streams(ctx)) != P2Z_OK) return r;
-    int32_t kbits;
-    std::memcpy(&kbits, &pl.kfact, sizeof kbits);
-    std::vector<int64_t> key = {pl.B, pl.nlayer, pl.niter, kbits, pl.upd, pl.sc, pl.block, pl.tpt, (int64_t)pl.flags,
-                                pl.nbatches, pl.soa, pl.uneven, schedule, user_mask,
-                                (int64_t)(uintptr_t)trk_in, (int64_t)(uintptr_t)hits, (int64_t)(uintptr_t)hit_mask,
-                                (int64_t)(uintptr_t)trk_out, (int64_t)(uintptr_t)ctx->trk.p,
-                                (int64_t)(uintptr_t)ctx->hits.p, (int64_t)(uintptr_t)ctx->out.p,
-                                (int64_t)(uintptr_t)ctx->mask.p, (int64_t)(uintptr_t)d_mask};
-    key.insert(key.end(), pl.ev_slot_begin.begin(), pl.ev_slot_begin.end());
-    if (!(ctx->run_exec && ctx->run_key == key)) {
-      if (ctx->run_exec) cudaGraphExecDestroy(ctx->run_exec);
-      ctx->run_exec = nullptr;
-      ctx->run_key.clear();
-      P2Z_CUDA(ctx, cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
-      r = pipeline();
-      cudaGraph_t g = nullptr;
-      const cudaError_t e = cudaStreamEndCapture(s0, &g);
-      if (r != P2Z_OK || e != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        cudaGetLastError();
-        return r != P2Z_OK ? r : fail(ctx, P2Z_CUDA_ERROR, "recording p2z_run's pipeline: %s", cudaGetErrorString(e));
-      }
-      const cudaError_t e2 = cudaGraphInstantiate(&ctx->run_exec, g, 0);
-      cudaGraphDestroy(g);
-      if (e2 != cudaSuccess) {
-        ctx->run_exec = nullptr;
-        return fail(ctx, P2Z_CUDA_ERROR, "cudaGraphInstantiate: %s", cudaGetErrorString(e2));
-      }
-      ctx->run_key = std::move(key);
-      ctx->run_launches = launches;
-      ctx->run_h2d = h2d;
-      ctx->run_d2h = d2h;
-    }
-    launches = ctx->run_launches;
-    h2d = ctx->run_h2d;
-    d2h = ctx->run_d2h;
-    P2Z_CUDA(ctx, cudaEventRecord(ctx->ev0, s0));
-    P2Z_CUDA(ctx, cudaGraphLaunch(ctx->run_exec, s0));
-  } else {
-    P2Z_CUDA(ctx, cudaEventRecord(ctx->ev0, s0));
-    if ((r = pipeline()) != P2Z_OK) return r;
   }
-  P2Z_CUDA(ctx, cudaEventRecord(ctx->ev1, s0));
+  P2Z_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, sp));
+  P2Z_CUDA(ctx, cudaEventRecord(ctx->ev1, sp));
   P2Z_CUDA(ctx, cudaEventSynchronize(ctx->ev1));
   const unsigned int status = *(volatile unsigned int *)ctx->h_status;  // copied by the pipeline's last step
   if (stats) {
@@ -987,7 +946,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
     stats->d2h_bytes = d2h;
     stats->launches = launches;
     stats->singular = (status & 1u) ? 1 : 0;
-    r = count_updates(ctx, pl, d_mask, s0, &stats->updates);
+    r = count_updates(ctx, pl, d_mask, sp, &stats->updates);
     if (r != P2Z_OK) return r;
   }
   if (status & 4u) return fail(ctx, P2Z_NONFINITE_INPUT, "a track or hit word the pass read is NaN or Inf");
