@@ -35,11 +35,11 @@ constexpr int kEventStreams = 10;
 // Threads per CTA where neither the caller nor the autotuner says: flat launches
 // take CTAs of one warp, which leave their registers as soon as the warp is done
 // (one B200, us per pass with 32 / 128: 1000 x 9600 tracks 1646 / 1651, 500 masked
-// events 606 / 610, 60 with the FP64 island sorted 161 / 168).  The FP32 kinds on
-// sorted windows take the window's four warps as one CTA: they read the same
-// sectors of hits, which one SM's L1 then holds for all of them (500 masked
-// events, under the power cap that a longer load meets, 627 / 577).  The queue
-// kernels' warps fetch their next work themselves.
+// events in stored order 606 / 610).  Sorted windows take the window's four warps
+// as one CTA: they read the same sectors of hits, which one SM's L1 then holds for
+// all of them (500 masked events, under the power cap that a longer load meets,
+// 627 / 577, 60 with the 3-D update 143 / 139).  The queue kernels' warps fetch their
+// next work themselves.
 constexpr int kFlatBlock = 32, kSortedBlock = p2z::kSortWindow, kQueueBlock = 128;
 namespace p2z {
 cudaError_t launch_step(int bsize, float *trk, const float *hits, int64_t nslots, int nlayer, int layer, int what,
@@ -362,7 +362,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   const bool sort = spec.masked && !padded && (pl.flags & P2Z_FLAG_SORT_WINDOWS) &&
                     (schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PERSISTENT);
   spec.args.sort = sort ? 1 : 0;
-  if (sort && !pl.block) spec.block = pl.upd == UPDK_3X3_F64 || pl.upd == UPDK_F64 ? kFlatBlock : kSortedBlock;
+  if (sort && !pl.block) spec.block = kSortedBlock;
   if (schedule == P2Z_SCHED_FLAT || sort) {
     spec.kind = KIND_FLAT;
     spec.duo = duo_mode(spec, padded, pl.host ? 0 : ctx->num_sms);

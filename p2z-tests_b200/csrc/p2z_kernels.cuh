@@ -271,10 +271,47 @@ __device__ __forceinline__ bool step(Trk<typename Types<UPD>::T, typename Types<
   }
 }
 
+// Rings of hits in shared memory, filled by asynchronous copies up to a stage less
+// than the ring ahead of the step that reads them (one commit group a step).
+__device__ __forceinline__ void copy_async_16(uint32_t dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int STAGES>
+__device__ __forceinline__ void copy_wait() {  // all but the newest STAGES - 2 groups have arrived
+  asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+}
+__device__ __forceinline__ uint32_t shared_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void copy_async_4(uint32_t dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// The masked 3-D kernels' ring: a lane's own words of its next present layers.
+// Lanes at different layers, and sorted windows more so, touch many sectors a
+// load; at 9 words a layer and 16 warps an SM the next layer in registers did not
+// cover that (one B200, 60 masked events, sorted, us per pass: registers 147, a
+// ring of 3 or 4 stages 139).  The 2-D kernels' 24 warps do without (500 masked
+// events, under the power cap: 569 with registers, 577 with the ring).
+constexpr int kMaskedRing = 3;
+template <int UPD, bool MASKED, int TPT>
+constexpr bool uses_ring() { return MASKED && TPT == 1 && Types<UPD>::NH == 9; }
+template <int UPD>
+constexpr int masked_ring_words() { return kMaskedRing * Types<UPD>::NH * 32; }  // a warp
+
+// Programmatic dependent launch (LaunchSpec::early).  This launch may have been set
+// up while the one in front of it ran, and touches no memory before that one is
+// complete.  Before its tracks' stores a thread lets the next launch be set up: no
+// earlier, since CTAs that wait on an SM take the place of running ones (with
+// the next launch let in at the start, 64,000 tracks took 27.1 us where they take
+// 19.1), no later, so that the set-up hides behind the stores.  Without the
+// attribute both do nothing.  One B200, passes queued behind one another, us each,
+// with / without: one event of 1024 tracks 7.9 / 10.2, 64 x 4096 tracks 54.2 / 57.3.
+__device__ __forceinline__ void start_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // Process one track slot: load, run every present layer, store.  TPT = 2: both
 // lanes of the pair load the track and its hits, and lane 0 stores the result.
 template <int B, int UPD, int SC, bool MASKED, int TPT = 1>
-__device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot) {
+__device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot, float *ring = nullptr) {
   using T = typename Types<UPD>::T;
   using A = typename Types<UPD>::A;
   constexpr int NH = Types<UPD>::NH;
@@ -290,6 +327,28 @@ __device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot) {
   const bool writer = TPT == 1 || !ln.j;
   const uint32_t all = (a.nlayer >= 32) ? 0xffffffffu : ((1u << a.nlayer) - 1u);
   uint32_t m = MASKED ? (__ldg(a.mask + slot) & all) : all;
+  // the ring's copies start before the track's words are needed
+  constexpr bool RING = uses_ring<UPD, MASKED, TPT>();
+  uint32_t todo = m, ring_dst = 0u;
+  const float *ring_src = nullptr;
+  int fill = 0;
+  auto copy = [&]() {  // the next present layer's hits
+    if (todo) {
+      const float *p = ring_src + (__ffs(todo) - 1) * (HIT_WORDS * WS);
+      todo &= todo - 1u;
+      const uint32_t d = ring_dst + fill * (NH * 128);
+#pragma unroll
+      for (int e = 0; e < NH; ++e) copy_async_4(d + e * 128, p + e * WS);
+    }
+    copy_commit();
+    fill = (fill + 1) % kMaskedRing;
+  };
+  if constexpr (RING) {
+    ring_dst = shared_u32(ring) + (threadIdx.x & 31) * 4;
+    ring_src = hit_lane<B>(a.hits, slot, a.nlayer, 0, WS);
+#pragma unroll
+    for (int i = 0; i < kMaskedRing - 1; ++i) copy();
+  }
   if constexpr (B > 0) {
     if (a.l2_prefetch && m != 0u) prefetch_hits_l2<B>(a.hits, slot, a.nlayer);
   }
@@ -373,6 +432,23 @@ __device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot) {
       singular |= step<UPD, SC, false, TPT>(s, b21, h0, k, ik, ln);
     }
     if (l < nl) singular |= step<UPD, SC, false, TPT>(s, b21, h1, k, ik, ln);
+  } else if constexpr (RING) {
+    const float *mine = ring + (threadIdx.x & 31);
+    int at = 0;
+    auto take = [&]() {
+      copy_wait<kMaskedRing>();
+#pragma unroll
+      for (int e = 0; e < NH; ++e) h0.w[e] = mine[at * (NH * 32) + e * 32];
+      at = (at + 1) % kMaskedRing;
+      copy();
+    };
+    take();
+    singular |= step<UPD, SC, true, TPT>(s, b21, h0, k, ik, ln);
+#pragma unroll 1
+    for (uint32_t rest = m & (m - 1u); rest; rest &= rest - 1u) {
+      take();
+      singular |= step<UPD, SC, false, TPT>(s, b21, h0, k, ik, ln);
+    }
   } else {
     // present layers in order: lowest set bit first
     const int64_t stride = HIT_WORDS * WS;
@@ -392,6 +468,7 @@ __device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot) {
     }
   }
 
+  let_next_start();
   const float z0 = 0.0f;
   float o[TRK_WORDS];
   o[0] = tof(s.x); o[1] = tof(s.y); o[2] = float(s.z);
@@ -413,17 +490,6 @@ __device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot) {
 
 
 
-// Programmatic dependent launch (LaunchSpec::early): this launch may have been set
-// up while the one in front of it ran, and touches no memory before that one is
-// complete; then (so that no more than one launch waits on the SMs) it lets the
-// next one be set up.  Without the attribute both do nothing.  One B200, passes
-// over one event of 1024 tracks queued behind one another: 8.1 us each, 10.2
-// without; 64 x 4096 tracks 54.6 and 57.3.
-__device__ __forceinline__ void start_after_previous() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
-}
-
 // One launch over slots [slot_begin, slot_end), TPT threads per slot.
 template <int B, int UPD, int SC, bool MASKED, int TPT = 1>
 __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_flat(RunArgs a) {
@@ -439,7 +505,8 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_flat(RunArgs a) {
     }
   }
   if (slot >= a.slot_end) return;  // (both lanes of a pair together)
-  process_slot<B, UPD, SC, MASKED, TPT>(a, slot);
+  extern __shared__ __align__(16) float hit_ring[];
+  process_slot<B, UPD, SC, MASKED, TPT>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
 }
 
 // Persistent launch: grid = resident CTAs; each warp repeatedly takes the next
@@ -449,6 +516,7 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_flat(RunArgs a) {
 template <int B, int UPD, int SC, bool MASKED, int TPT = 1>
 __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_persistent(RunArgs a) {
   constexpr int kPer = 32 / TPT;  // slots per work item
+  extern __shared__ __align__(16) float hit_ring[];
   const int lane = threadIdx.x & 31;
   const int64_t nslots = a.slot_end - a.slot_begin;
   const unsigned long long nitems = (unsigned long long)((nslots + kPer - 1) / kPer);
@@ -458,7 +526,8 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_persistent(RunArg
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= nitems) break;
     const int64_t slot = a.slot_begin + (int64_t)item * kPer + lane / TPT;
-    if (slot < a.slot_end) process_slot<B, UPD, SC, MASKED, TPT>(a, slot);
+    if (slot < a.slot_end)
+      process_slot<B, UPD, SC, MASKED, TPT>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
   }
 }
 
@@ -484,13 +553,6 @@ constexpr int kDuoRing = 4;
 constexpr int kDuoStage = 6 * 64;  // words
 constexpr int duo_smem_bytes(int threads) { return threads / 32 * kDuoRing * kDuoStage * 4; }
 
-__device__ __forceinline__ void copy_async_16(uint32_t dst, const float *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// All but the newest kDuoRing - 2 groups have arrived.
-__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kDuoRing - 2) : "memory"); }
-__device__ __forceinline__ uint32_t shared_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 template <bool GENERAL>
 __device__ __forceinline__ bool step_duo(Trk<float2, APT<float2>> &s, const float2 *b21, const HitPair &h, float2 k,
@@ -596,7 +658,7 @@ __device__ __forceinline__ void process_duo(const RunArgs &a, int64_t w0, float 
   bool singular = false;
   const float2 *mine = reinterpret_cast<const float2 *>(ring + own / ROW * (6 * ROW) + own % ROW);
   auto take = [&](HitPair &h, int l) {  // layer l's hits, then the copy that refills the stage before it
-    copy_wait();
+    copy_wait<kDuoRing>();
     __syncwarp();
     const float2 *at = mine + l % kDuoRing * (kDuoStage / 2);
 #pragma unroll
@@ -611,6 +673,7 @@ __device__ __forceinline__ void process_duo(const RunArgs &a, int64_t w0, float 
     take(h, l);
     singular |= step_duo<false>(s, nullptr, h, k, ik, live);
   }
+  let_next_start();
   if (!valid) return;
   float2 o[TRK_WORDS];
   finish_duo(s, q, o);
@@ -1006,6 +1069,8 @@ struct Dispatch {
   }
   // dynamic shared memory of a launch
   static size_t smem_bytes(const LaunchSpec &s) {
+    if (s.masked && uses_ring<UPD, true, 1>() && s.kind != KIND_STAGED)
+      return (size_t)(s.block / 32) * masked_ring_words<UPD>() * sizeof(float);
     if (s.duo >= 0) return duo_smem_bytes(std::min(s.block, kDuoThreads));
     return s.kind == KIND_STAGED ? (size_t)(s.block / 32) * StagedSmem<UPD>::kWarpBytes : 0;
   }
