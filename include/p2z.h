@@ -120,9 +120,7 @@ typedef enum p2z_update_kind {
 /* How the work is laid onto the GPU.
  *  AUTO        FLAT; with a caller's hit mask and enough slots to fill the GPU more than once, FLAT
  *              with P2Z_FLAG_SORT_WINDOWS.
- *  FLAT        one launch over every track slot of every event (P2Z_UPDATE_V2 without missing
- *              layers and without P2Z_FLAG_ACCURATE_TRIG or REFERENCE_ROUNDING, on 16-byte
- *              aligned arrays: two tracks per thread when the launch fills the GPU).
+ *  FLAT        one launch over every track slot of every event.
  *  PER_EVENT   one launch per event (the reference's launch-per-chunk form,
  *              src/propagate-toz-test_CUDA_v4.cu:970-986, taken down to one event per launch).
  *  PERSISTENT  one persistent launch (grid = resident CTAs) whose warps take
@@ -210,13 +208,13 @@ typedef struct p2z_config {
                             this context for the same key, else the rule under p2z_schedule */
   int32_t block_threads; /* threads per CTA, a multiple of 32 in 32..256; 0 -> the value
                             p2z_autotune measured best on this context for the same update,
-                            flags, bsize, layout and masking, else 32 (FLAT, PER_EVENT) or 128;
-                            the two-tracks-per-thread form uses at most 128 */
+                            flags, bsize, layout and masking, else 32 (FLAT, PER_EVENT),
+                            128 (other schedules, sorted windows) */
   uint32_t flags;        /* P2Z_FLAG_*; any other bit is P2Z_BAD_ARG */
   int32_t layout;        /* p2z_layout of the track, hit and output arrays */
   /* Uneven form (optional, host memory): nevts track counts.  NULL -> uniform. */
   const int64_t *event_ntrks;
-  int32_t threads_per_track; /* 1 (a thread may hold two tracks, see P2Z_SCHED_FLAT), or 2 (P2Z_UPDATE_V2 without REFERENCE_ROUNDING; FLAT,
+  int32_t threads_per_track; /* 1, or 2 (P2Z_UPDATE_V2 without REFERENCE_ROUNDING; FLAT,
                             PER_EVENT and PERSISTENT schedules): lanes 2i and 2i+1 of a warp
                             hold the same track and split the propagation of its covariance,
                             with bit-identical results.  0 -> the value p2z_autotune measured

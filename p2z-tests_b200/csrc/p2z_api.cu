@@ -25,8 +25,8 @@ constexpr int64_t kRunMinBatches = 64, kRunMinShare = 64;
 // That reaches 50 GB/s in where the copies reach 55, but has no chunk to fill before
 // the first track and none to drain after the last, and copies in and out that
 // meet slow each other by 20-40 us a piece.  One B200, wall us a call, copies (the
-// best of 4-16 chunks) / direct: 1024 tracks 64 / 49, 9600 189 / 157, 16 x 9600 (91 MB)
-// 1954 / 1879, 64 x 9600 (364 MB) 7230 / 7274.  Batches narrower than 32 slots write
+// best of 4-16 chunks) / direct: 1024 tracks 64 / 58, 9600 189 / 159, 16 x 9600 (91 MB)
+// 1954 / 1892, 64 x 9600 (364 MB) 7230 / 7274.  Batches narrower than 32 slots write
 // less than 128 bytes at a time (bsize 8: 2295 / 3524).
 constexpr size_t kRunDirectBytes = size_t(256) << 20;
 constexpr int kRunMaxChunks = 16;  // ln(64)/ln(3/2) + 1 of them at most, and the rest taken whole
@@ -34,7 +34,7 @@ constexpr int kRunMaxChunks = 16;  // ln(64)/ln(3/2) + 1 of them at most, and th
 constexpr int kEventStreams = 10;
 // Threads per CTA where neither the caller nor the autotuner says: flat launches
 // take CTAs of one warp, which leave their registers as soon as the warp is done
-// (one B200, us per pass with 32 / 128: 1000 x 9600 tracks 1646 / 1651, 500 masked
+// (one B200, us per pass with 32 / 128: 100 x 9600 tracks 188.5 / 194.6, 500 masked
 // events in stored order 606 / 610).  Sorted windows take the window's four warps
 // as one CTA: they read the same sectors of hits, which one SM's L1 then holds for
 // all of them (500 masked events, under the power cap that a longer load meets,
@@ -315,7 +315,6 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   spec.block = pl.block ? pl.block : (flat ? kFlatBlock : kQueueBlock);
   spec.grid = 0;
   spec.tpt = pl.tpt;
-  spec.duo = -1;
   spec.early = flat && pl.early;
   const bool padded = base.mask != nullptr && base.mask == pl.padding_mask;
   // Launches of at most 4 warps per SM leave each scheduler about one warp, with
@@ -342,7 +341,6 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
       spec.args.slot_begin = a;
       spec.args.slot_end = b;
       spec.args.l2_prefetch = prefetch_for(b - a);
-      spec.duo = duo_mode(spec, padded, pl.host ? 0 : ctx->num_sms);
       P2Z_CUDA(ctx, dispatch(spec, spread ? ctx->ev_streams[k++ % kEventStreams] : st));
       ++*launches;
     }
@@ -365,7 +363,6 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   if (sort && !pl.block) spec.block = kSortedBlock;
   if (schedule == P2Z_SCHED_FLAT || sort) {
     spec.kind = KIND_FLAT;
-    spec.duo = duo_mode(spec, padded, pl.host ? 0 : ctx->num_sms);
     P2Z_CUDA(ctx, dispatch(spec, st));
     ++*launches;
     return P2Z_OK;

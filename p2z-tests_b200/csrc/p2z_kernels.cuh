@@ -237,45 +237,41 @@ __device__ __forceinline__ bool step(Trk<typename Types<UPD>::T, typename Types<
   Jac<T> J;
   if constexpr (UPD == UPDK_F64) {
     hx = propagate_params_f64(s, zout, k);
-    J = jacobian_f64(hx, k, s.ipt, GENERAL);
+    J = jacobian_precise<double, GENERAL>(hx, k, s.ipt);
   } else if constexpr (UPD == UPDK_V2_REF) {
     hx = propagate_params_ref(s, zout, k);
     J = jacobian_ref(hx, k, s.ipt);
   } else {
-    hx = propagate_params_precise<SC>(s, zout, k, ik, true);
-    J = jacobian_precise<GENERAL>(hx, k, s.ipt);
+    hx = propagate_params_precise<SC>(s, zout, k, ik);
+    J = jacobian_precise<float, GENERAL>(hx, k, s.ipt);
   }
-  if constexpr (UPD == UPDK_F64 || UPD == UPDK_V2_REF) {
-    if constexpr (GENERAL) propagate_cov_general(s, b21, J);
-    else propagate_cov_reduced(s, J);
-  } else {
-    if constexpr (GENERAL) propagate_cov_general_precise(s, b21, J);
-    else if constexpr (TPT == 2) propagate_cov_reduced_pair(s, J, ln.j, ln.pm);
-    else propagate_cov_precise(s, J);
-  }
+  if constexpr (GENERAL) propagate_cov_general(s, b21, hx, J);
+  else if constexpr (TPT == 2) propagate_cov_reduced_pair(s, J, ln.j, ln.pm);
+  else if constexpr (P2Z_PACKED_F32X2 && std::is_same<T, float>::value && UPD != UPDK_V2_REF)
+    propagate_cov_reduced_packed(s, J);  // (the reference-rounding form keeps separate roundings)
+  else propagate_cov_reduced(s, J);
   if constexpr (UPD == UPDK_F64) {
     const double hp[3] = {h.w[0], h.w[1], h.w[2]};
     const double hc[3] = {h.w[3], h.w[4], h.w[5]};
     return update_v2_f64(s, hp, hc);
-  } else if constexpr (UPD == UPDK_V2_REF) {
-    const float hp[3] = {h.w[0], h.w[1], h.w[2]};
-    const float hc[3] = {h.w[3], h.w[4], h.w[5]};
-    return update_v2_ref(s, hp, hc);
-  } else if constexpr (UPD == UPDK_V2 || UPD == UPDK_V2_COMP) {
-    return update_v2_precise<GENERAL>(s, h.w[0], h.w[1], h.w[3], h.w[4], h.w[5], true);
   } else {
     const float hp[3] = {h.w[0], h.w[1], h.w[2]};
-    const float hv[6] = {h.w[3], h.w[4], h.w[5], h.w[6], h.w[7], h.w[8]};
-    if constexpr (UPD == UPDK_3X3_F64) return update_3x3_joseph<double>(s, hp, hv);
-    else return update_3x3_joseph<float>(s, hp, hv);
+    if constexpr (UPD == UPDK_V2 || UPD == UPDK_V2_REF) {
+      const float hc[3] = {h.w[3], h.w[4], h.w[5]};
+      return update_v2<typename Types<UPD>::A, (UPD == UPDK_V2_REF) ? FORM_REFERENCE : FORM_PRECISE, GENERAL>(s, hp, hc);
+    } else if constexpr (UPD == UPDK_V2_COMP) {
+      const float hc[3] = {h.w[3], h.w[4], h.w[5]};
+      return update_v2<DF, FORM_PRECISE, GENERAL>(s, hp, hc);
+    } else {
+      const float hv[6] = {h.w[3], h.w[4], h.w[5], h.w[6], h.w[7], h.w[8]};
+      if constexpr (UPD == UPDK_3X3_F64) return update_3x3_joseph<double>(s, hp, hv);
+      else return update_3x3_joseph<float>(s, hp, hv);
+    }
   }
 }
 
 // Rings of hits in shared memory, filled by asynchronous copies up to a stage less
 // than the ring ahead of the step that reads them (one commit group a step).
-__device__ __forceinline__ void copy_async_16(uint32_t dst, const float *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int STAGES>
 __device__ __forceinline__ void copy_wait() {  // all but the newest STAGES - 2 groups have arrived
@@ -529,184 +525,6 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_persistent(RunArg
     if (slot < a.slot_end)
       process_slot<B, UPD, SC, MASKED, TPT>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
   }
-}
-
-// ---------------------------------------------------------------------------
-// Two tracks per thread (UPDK_V2, SC_FAST): a thread holds the tracks of two
-// slots in the two halves of packed FP32x2 registers, so that every
-// floating-point instruction of the step works on both -- the one-track kernel
-// can pair only the two measured rows of one track.
-// ---------------------------------------------------------------------------
-// How the layers of a launch's tracks are given: DUO_ALL every slot has every
-// layer, DUO_PADDED every slot has every layer or is padding (the library's own
-// mask of uneven events).
-enum { DUO_ALL = 0, DUO_PADDED = 1 };
-
-struct HitPair {
-  float2 w[6];
-};
-
-// The hits stream through a ring of kDuoRing shared-memory stages a warp, a
-// stage holding one step's 6 words of its 64 tracks, filled by asynchronous
-// copies up to kDuoRing - 1 steps ahead.
-constexpr int kDuoRing = 4;
-constexpr int kDuoStage = 6 * 64;  // words
-constexpr int duo_smem_bytes(int threads) { return threads / 32 * kDuoRing * kDuoStage * 4; }
-
-
-template <bool GENERAL>
-__device__ __forceinline__ bool step_duo(Trk<float2, APT<float2>> &s, const float2 *b21, const HitPair &h, float2 k,
-                                         float2 ik, Bool2 live) {
-  const Helix<float2> hx = propagate_params_precise<SC_FAST>(s, h.w[2], k, ik, live);
-  const Jac<float2> J = jacobian_precise<GENERAL>(hx, k, s.ipt);
-  if constexpr (GENERAL) propagate_cov_general_precise(s, b21, J);
-  else propagate_cov_precise(s, J);
-  return update_v2_precise<GENERAL>(s, h.w[0], h.w[1], h.w[3], h.w[4], h.w[5], live);
-}
-
-__device__ __forceinline__ void start_duo(Trk<float2, APT<float2>> &s, const float2 (&in)[TRK_WORDS], float kfact,
-                                          float2 &k, float2 &ik) {
-  k = make_float2(float(__float_as_int(in[27].x)) * kfact, float(__float_as_int(in[27].y)) * kfact);
-  ik = make_float2(1.f / k.x, 1.f / k.y);
-  acc_set(s.x, in[0]);
-  acc_set(s.y, in[1]);
-  s.phi = in[4];
-  s.z = in[2]; s.ipt = in[3]; s.theta = in[5];
-  init_direction(s);
-}
-
-// The output words of a track pair, in the order of the arrays.
-__device__ __forceinline__ void finish_duo(const Trk<float2, APT<float2>> &s, float2 q, float2 (&o)[TRK_WORDS]) {
-  const float2 z0 = make_float2(0.f, 0.f);
-  o[0] = vadd(s.x.a, s.x.u); o[1] = vadd(s.y.a, s.y.u); o[2] = s.z;
-  o[3] = s.ipt; o[4] = s.phi; o[5] = s.theta;
-  float2 *c = o + 6;
-  c[0] = s.c00; c[1] = s.c10; c[2] = s.c11;
-  c[3] = z0; c[4] = z0; c[5] = z0;
-  c[6] = s.c30; c[7] = s.c31; c[8] = z0; c[9] = s.c33;
-  c[10] = s.c40; c[11] = s.c41; c[12] = z0; c[13] = s.c43; c[14] = s.c44;
-  c[15] = s.c50; c[16] = s.c51; c[17] = z0; c[18] = s.c53; c[19] = s.c54; c[20] = s.c55;
-  o[27] = q;
-}
-
-// Slots slot and slot + 1 (slot even: the same batch, neighbouring words), with
-// every layer; DUO_PADDED: of a slot that is padding the track passes through.
-// The warp's 64 slots (w0 on) hold 6 rows of hits a layer, 1536 bytes, copied in
-// 96 pieces of 16 bytes, three a lane.  A lane past the launch's end works on
-// the last slots again and stores nothing.
-template <int B, int MODE>
-__device__ __forceinline__ void process_duo(const RunArgs &a, int64_t w0, float *ring) {
-  constexpr int ROW = (B > 0 && B < 64) ? B : 64;  // neighbouring slots of a row of hit words
-  const int64_t WS = (B > 0) ? (int64_t)B : a.ws;
-  const int lane = threadIdx.x & 31;
-  const int have = (int)min((int64_t)64, a.slot_end - w0);  // a multiple of 8
-  const int own = min(2 * lane, have - 2);
-  const bool valid = 2 * lane < have;
-  const int64_t slot = w0 + own;
-  const int64_t stride = HIT_WORDS * WS;
-  const int nl = a.nlayer;
-  // this lane's pieces: piece p covers 4 words of row (p / (ROW/4)) % 6 of the
-  // (p / (6 ROW/4))-th group of ROW slots
-  const float *src[3];
-  bool has[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const int p = lane + 32 * j;
-    const int group = p / (6 * ROW / 4), row = p / (ROW / 4) % 6, at = group * ROW + p % (ROW / 4) * 4;
-    has[j] = at < have;
-    src[j] = hit_lane<B>(a.hits, w0 + (has[j] ? at : 0), nl, 0, WS) + row * WS;
-  }
-  const uint32_t dst = shared_u32(ring) + lane * 16;
-  int fill = 0;  // stage of the next copy
-  auto copy = [&](int l) {
-    if (l < nl) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        if (has[j]) copy_async_16(dst + (fill * kDuoStage + j * 128) * 4, src[j]);
-        src[j] += stride;
-      }
-    }
-    copy_commit();
-    fill = (fill + 1) % kDuoRing;
-  };
-#pragma unroll
-  for (int l = 0; l < kDuoRing - 1; ++l) copy(l);
-
-  const float *tin = trk_lane<B>(a.trk, slot);
-  float *tout = const_cast<float *>(trk_lane<B>(a.out, slot));
-  Bool2 live = {true, true};
-  if constexpr (MODE == DUO_PADDED) {
-    const uint2 m = __ldg(reinterpret_cast<const uint2 *>(a.mask + slot));
-    live = {m.x != 0u, m.y != 0u};
-  }
-  float2 in[TRK_WORDS];
-#pragma unroll
-  for (int e = 0; e < TRK_WORDS; ++e) in[e] = __ldg(reinterpret_cast<const float2 *>(tin + e * WS));
-  if constexpr (MODE == DUO_PADDED) {
-    if (valid && !(live.x && live.y)) {
-#pragma unroll
-      for (int e = 0; e < TRK_WORDS; ++e) {
-        if (!live.x) __stcs(tout + e * WS, in[e].x);
-        if (!live.y) __stcs(tout + e * WS + 1, in[e].y);
-      }
-    }
-  }
-  Trk<float2, APT<float2>> s;
-  float2 k, ik;
-  start_duo(s, in, a.kfact, k, ik);
-  const float2 q = in[27];
-  bool singular = false;
-  const float2 *mine = reinterpret_cast<const float2 *>(ring + own / ROW * (6 * ROW) + own % ROW);
-  auto take = [&](HitPair &h, int l) {  // layer l's hits, then the copy that refills the stage before it
-    copy_wait<kDuoRing>();
-    __syncwarp();
-    const float2 *at = mine + l % kDuoRing * (kDuoStage / 2);
-#pragma unroll
-    for (int e = 0; e < 6; ++e) h.w[e] = at[e * (ROW / 2)];
-    copy(l + kDuoRing - 1);
-  };
-  HitPair h;
-  take(h, 0);
-  singular |= step_duo<true>(s, in + 6, h, k, ik, live);
-#pragma unroll 1
-  for (int l = 1; l < nl; ++l) {
-    take(h, l);
-    singular |= step_duo<false>(s, nullptr, h, k, ik, live);
-  }
-  let_next_start();
-  if (!valid) return;
-  float2 o[TRK_WORDS];
-  finish_duo(s, q, o);
-  if (MODE == DUO_ALL || (live.x && live.y)) {
-#pragma unroll
-    for (int e = 0; e < TRK_WORDS; ++e) __stcs(reinterpret_cast<float2 *>(tout + e * WS), o[e]);
-  } else if (live.x || live.y) {
-#pragma unroll
-    for (int e = 0; e < TRK_WORDS; ++e) __stcs(tout + e * WS + (live.x ? 0 : 1), live.x ? o[e].x : o[e].y);
-  }
-  if (singular) atomicOr(a.status, 1u);
-}
-
-// What bounds it: register reads.  A scheduler's register file delivers two
-// operands a lane and cycle, so a packed multiply-add of three register pairs
-// takes 3 cycles (measured: 2.97; with a constant operand 2.01, with one half
-// broadcast 2.49), a scalar one 1.5, and both kernels run at that limit.  Two
-// tracks per thread leave the arithmetic's reads as they are and halve those of
-// everything else (addresses, loads, stores, loop and branches), 150 against 260
-// instructions a track-step.  148 registers: 12 warps of 64 tracks an SM, as many
-// tracks in flight as the one-track kernel's 24 warps of 32 (a cap of 128, 16
-// warps, spills 32 bytes and is 1-3% slower).  So few warps do not hide a layer's
-// latency, hence the ring.  One B200, 20 layers, us per pass, one-track kernel /
-// this: 1000 x 9600 tracks 1772 / 1646, 100 x 9600 186.5 / 174.3, 64 x 4096 SoA
-// 66.3 / 57.1; this one with the next layer prefetched into registers instead of
-// the ring 181.4 and 62.6 on the last two.
-constexpr int kDuoThreads = 128;
-template <int B, int MODE>
-__global__ void __launch_bounds__(kDuoThreads, 3) k_duo(RunArgs a) {
-  start_after_previous();
-  extern __shared__ __align__(16) float duo_ring[];
-  const int64_t w0 = a.slot_begin + 64 * (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (w0 < a.slot_end) process_duo<B, MODE>(a, w0, duo_ring + (threadIdx.x >> 5) * (kDuoRing * kDuoStage));
 }
 
 // ---------------------------------------------------------------------------
@@ -1006,7 +824,6 @@ struct LaunchSpec {
   int block;     // threads per CTA
   int grid;      // CTAs (persistent); flat computes its own
   int tpt;       // threads per track: 1, or 2 (UPDK_V2, flat and persistent kinds)
-  int duo;       // two tracks per thread (duo_mode): DUO_*, or -1
   bool early;    // flat kinds: programmatic dependent launch
 };
 
@@ -1029,23 +846,6 @@ int occupancy_3x3_f64(const LaunchSpec &s);
 int occupancy_3x3_comp(const LaunchSpec &s);
 int occupancy_f64(const LaunchSpec &s);
 int occupancy_v2_ref(const LaunchSpec &s);
-
-// The two-tracks-per-thread form a launch takes (DUO_*), or -1: the precise 2-D
-// update on flat launches without missing layers, big enough to fill the GPU --
-// below kDuoMinSlotsPerSm slots an SM the one-track kernel's twice as many warps
-// finish sooner -- whose arrays the 8- and 16-byte accesses can reach (SoA rows
-// and bsizes are multiples of 8 words).  padded: the mask is the library's own.
-// One B200, 20 layers, us per pass, one-track kernel / this: 57,600 tracks 20.5 /
-// 18.5, 76,800 24.7 / 26.1, 96,000 28.8 / 26.7, 192,000 47.1 / 45.1.
-constexpr int64_t kDuoMinSlotsPerSm = 640;
-inline int duo_mode(const LaunchSpec &s, bool padded, int num_sms) {
-  const RunArgs &a = s.args;
-  if (s.upd != UPDK_V2 || s.sc != SC_FAST || s.tpt != 1 || s.kind != KIND_FLAT || (a.mask && !padded)) return -1;
-  if (a.slot_end - a.slot_begin < (int64_t)num_sms * kDuoMinSlotsPerSm) return -1;
-  if ((a.slot_begin | a.slot_end | a.ws) & 7) return -1;
-  if (((uintptr_t)a.trk | (uintptr_t)a.hits | (uintptr_t)a.out | (uintptr_t)a.mask) & 15u) return -1;
-  return a.mask ? DUO_PADDED : DUO_ALL;
-}
 
 // Shared dispatch body: picks the template instance for (B, SC, MASKED, KIND,
 // threads per track).
@@ -1071,7 +871,6 @@ struct Dispatch {
   static size_t smem_bytes(const LaunchSpec &s) {
     if (s.masked && uses_ring<UPD, true, 1>() && s.kind != KIND_STAGED)
       return (size_t)(s.block / 32) * masked_ring_words<UPD>() * sizeof(float);
-    if (s.duo >= 0) return duo_smem_bytes(std::min(s.block, kDuoThreads));
     return s.kind == KIND_STAGED ? (size_t)(s.block / 32) * StagedSmem<UPD>::kWarpBytes : 0;
   }
   template <int B, int SC>
@@ -1085,27 +884,7 @@ struct Dispatch {
     }
     return fn_m<B, SC_ACCURATE>(masked, kind, tpt);
   }
-  template <int B>
-  static const void *fn_duo(int mode) {
-    if constexpr (HAS_PAIR) {
-      switch (mode) {
-        case DUO_ALL: return (const void *)k_duo<B, DUO_ALL>;
-        case DUO_PADDED: return (const void *)k_duo<B, DUO_PADDED>;
-      }
-    }
-    return nullptr;
-  }
   static const void *select(const LaunchSpec &s) {
-    if (s.duo >= 0) {
-      if (s.soa) return fn_duo<0>(s.duo);
-      switch (s.bsize) {
-        case 8: return fn_duo<8>(s.duo);
-        case 16: return fn_duo<16>(s.duo);
-        case 32: return fn_duo<32>(s.duo);
-        case 64: return fn_duo<64>(s.duo);
-        default: return nullptr;
-      }
-    }
     if (s.soa) return fn_sc<0>(s.sc, s.masked, s.kind, s.tpt);
     switch (s.bsize) {
       case 8: return fn_sc<8>(s.sc, s.masked, s.kind, s.tpt);
@@ -1120,13 +899,12 @@ struct Dispatch {
     if (!f) return cudaErrorInvalidValue;
     const int64_t slots = s.args.slot_end - s.args.slot_begin;
     if (slots <= 0) return cudaSuccess;
-    const int block = s.duo >= 0 ? std::min(s.block, kDuoThreads) : s.block;
     int grid;
     if (s.kind == KIND_PERSISTENT || s.kind == KIND_STAGED) {
       grid = s.grid;
     } else {
       const int64_t n = s.args.sort ? (slots + kSortWindow - 1) / kSortWindow * kSortWindow : slots;
-      grid = (int)(((s.duo >= 0 ? n / 2 : n * s.tpt) + block - 1) / block);
+      grid = (int)((n * s.tpt + s.block - 1) / s.block);
     }
     const size_t smem = smem_bytes(s);
     if (smem > 48 * 1024) {
@@ -1138,7 +916,7 @@ struct Dispatch {
     if (s.early) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(grid);
-      cfg.blockDim = dim3(block);
+      cfg.blockDim = dim3(s.block);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = st;
       cudaLaunchAttribute attr = {};
@@ -1148,7 +926,7 @@ struct Dispatch {
       cfg.numAttrs = 1;
       return cudaLaunchKernelExC(&cfg, f, params);
     }
-    return cudaLaunchKernel(f, dim3(grid), dim3(block), params, smem, st);
+    return cudaLaunchKernel(f, dim3(grid), dim3(s.block), params, smem, st);
   }
   static int occupancy(const LaunchSpec &s) {
     const void *f = select(s);

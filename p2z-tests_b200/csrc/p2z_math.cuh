@@ -68,12 +68,9 @@ struct DF {
 // step, so they round ~10x finer than the coordinate itself, and the Kalman
 // residual (h - a) - u is formed without cancellation error beyond the
 // rounding of h - a.  All FP32, full rate.
-// V: float, or float2 for two tracks in one thread.
-template <typename V>
-struct APT {
-  V a, u;
+struct AP {
+  float a, u;
 };
-using AP = APT<float>;
 
 __device__ __forceinline__ float tof(float v) { return v; }
 __device__ __forceinline__ float tof(AP v) { return v.a + v.u; }
@@ -84,8 +81,9 @@ __device__ __forceinline__ void acc_set(float &a, float v) { a = v; }
 __device__ __forceinline__ void acc_set(double &a, float v) { a = v; }
 __device__ __forceinline__ void acc_set(double &a, double v) { a = v; }
 __device__ __forceinline__ void acc_set(DF &a, float v) { a.hi = v; a.lo = 0.f; }
-template <typename V>
-__device__ __forceinline__ void acc_set(APT<V> &a, V v) { a.a = v; a.u = V(); }
+__device__ __forceinline__ void acc_set(AP &a, float v) { a.a = v; a.u = 0.f; }
+__device__ __forceinline__ void acc_add(AP &a, float d) { a.u += d; }
+
 // A float accumulator adds with an explicit rounding: an increment that is also
 // used elsewhere (the helix angle, the Kalman corrections of phi and theta) must
 // not be fused into the addition in one kernel and not in another, so that
@@ -123,87 +121,24 @@ __device__ __forceinline__ void acc_update(A &a, T h, T res, T inc) {
   acc_add(a, inc);
 }
 
+// Reciprocal: MUFU approximation refined by one Newton-Raphson step,
+// r' = r + r (1 - x r); within about 1 ulp of 1/x for normal x, no branch.
+__device__ __forceinline__ float rcp_nr(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float e = fmaf(-x, r, 1.0f);
+  return fmaf(r, e, r);
+}
+
 // Packed FP32 pairs: one sm_100 instruction performs two independent FP32
 // operations on a register pair (per component exactly __fmaf_rn / __fmul_rn),
 // halving the issue slots of paired arithmetic.
+#ifndef P2Z_PACKED_F32X2
+#define P2Z_PACKED_F32X2 1
+#endif
 __device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-
-// The precise form's arithmetic on V = float (one track a thread) or V = float2
-// (two tracks a thread, one per component).  Every operation is written with
-// its rounding, so that nothing is left to the compiler's contraction and a
-// track gets the same bits from every kernel.
-__device__ __forceinline__ float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ float vmul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ float vadd(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ float vsub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ float vneg(float a) { return -a; }
-__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __fadd2_rn(a, vneg(b)); }
-template <typename V>
-__device__ __forceinline__ V vset(float a) {
-  if constexpr (std::is_same<V, float2>::value) return make_float2(a, a);
-  else return a;
-}
-// per component: c ? a : b
-__device__ __forceinline__ float vsel(bool c, float a, float b) { return c ? a : b; }
-struct Bool2 {
-  bool x, y;
-};
-__device__ __forceinline__ float2 vsel(Bool2 c, float2 a, float2 b) {
-  return make_float2(c.x ? a.x : b.x, c.y ? a.y : b.y);
-}
-__device__ __forceinline__ bool vgt_abs(float a, float t) { return fabsf(a) > t; }
-__device__ __forceinline__ Bool2 vgt_abs(float2 a, float t) { return {fabsf(a.x) > t, fabsf(a.y) > t}; }
-
-__device__ __forceinline__ float vdiv(float a, float b) { return __fdiv_rn(a, b); }
-__device__ __forceinline__ float2 vdiv(float2 a, float2 b) { return make_float2(__fdiv_rn(a.x, b.x), __fdiv_rn(a.y, b.y)); }
-
-// -1/x: the MUFU approximation of the reciprocal refined by one Newton-Raphson
-// step, r' = r + r (1 - x r); within about 1 ulp for normal x, no branch.  (The
-// negative: its sign saves the products below their negations.)
-__device__ __forceinline__ float rcp_mufu(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float2 rcp_mufu(float2 x) { return make_float2(rcp_mufu(x.x), rcp_mufu(x.y)); }
-template <typename V>
-__device__ __forceinline__ V nrcp_nr(V x) {
-  const V r = rcp_mufu(vneg(x));
-  return vfma(r, vfma(x, r, vset<V>(1.f)), r);
-}
-
-// x += p*q on the position accumulators.
-template <typename V>
-__device__ __forceinline__ void acc_fma(APT<V> &a, V p, V q) {
-  a.u = vfma(p, q, a.u);
-}
-__device__ __forceinline__ void acc_fma(DF &a, float p, float q) { acc_add(a, __fmul_rn(p, q)); }
-
-// x - h, the negative of the Kalman residual.
-template <typename V>
-__device__ __forceinline__ V acc_nres(V h, const APT<V> &a) {
-  return vadd(vsub(a.a, h), a.u);
-}
-__device__ __forceinline__ float acc_nres(float h, const DF &a) { return -acc_res(h, a); }
-
-// After a Kalman update: nr = x - h, and the increment is nKs*nrs + nKo*nro
-// with s the coordinate itself and o the other one (nrs == nr).  AP re-anchors
-// at the hit, x + inc = h + (nr + inc): the sum starts from nr (1 + nKs), which
-// for a track the hit pins (K near 1) is the small difference itself.
-template <typename V>
-__device__ __forceinline__ void acc_kalman(APT<V> &a, V h, V nKs, V nrs, V nKo, V nro) {
-  a.a = h;
-  a.u = vfma(nKo, nro, vfma(nKs, nrs, nrs));
-}
-__device__ __forceinline__ void acc_kalman(DF &a, float, float nKs, float nrs, float nKo, float nro) {
-  acc_add(a, vfma(nKo, nro, vmul(nKs, nrs)));
-}
 
 // ---------------------------------------------------------------------------
 // sin / cos / versine
@@ -213,16 +148,15 @@ __device__ __forceinline__ void acc_kalman(DF &a, float, float nKs, float nrs, f
 // 1 - cos(a) = a^2/2! - a^4/4! + a^6/6! - a^8/8! (truncation below
 // a^10/10! ~ 2.2e-9 of the versine at |a| = 0.5).  The coefficients are
 // (-1)^n/(2n+1)! and (-1)^n/(2n)!, rounded to float.
-template <typename V>
-__device__ __forceinline__ void sv_series(V a, V *s, V *v) {
-  const V a2 = vmul(a, a);
-  V ps = vfma(a2, vset<V>(-1.9841270e-4f), vset<V>(8.3333333e-3f));
-  ps = vfma(a2, ps, vset<V>(-1.6666667e-1f));
-  *s = vfma(vmul(a, a2), ps, a);
-  V pv = vfma(a2, vset<V>(-2.4801587e-5f), vset<V>(1.3888889e-3f));
-  pv = vfma(a2, pv, vset<V>(-4.1666667e-2f));
-  pv = vfma(a2, pv, vset<V>(0.5f));
-  *v = vmul(a2, pv);
+__device__ __forceinline__ void sv_series(float a, float *s, float *v) {
+  const float a2 = a * a;
+  float ps = fmaf(a2, -1.9841270e-4f, 8.3333333e-3f);
+  ps = fmaf(a2, ps, -1.6666667e-1f);
+  *s = fmaf(a * a2, ps, a);
+  float pv = fmaf(a2, 2.4801587e-5f, -1.3888889e-3f);
+  pv = fmaf(a2, pv, 4.1666667e-2f);
+  pv = fmaf(a2, -pv, 0.5f);
+  *v = a2 * pv;
 }
 
 // tan(t + d) from tA = tan(t) and an offset d (the theta offset, which sums
@@ -234,14 +168,13 @@ __device__ __forceinline__ void sv_series(V a, V *s, V *v) {
 // 1.2e-8 absolute for |d| <= 0.2); the quotient is exact up to a Newton-refined
 // reciprocal.  The increment is formed first and added to tA last (one
 // rounding at the size of the result).
-template <typename V>
-__device__ __forceinline__ V tan_offset(V tA, V d) {
-  const V d2 = vmul(d, d);
-  V p = vfma(d2, vset<V>(5.3968254e-2f), vset<V>(1.3333334e-1f));
-  p = vfma(d2, p, vset<V>(3.3333334e-1f));
-  const V u = vfma(vmul(d, d2), p, d);
-  const V r = vmul(u, vfma(tA, tA, vset<V>(1.f)));
-  return vfma(r, vneg(nrcp_nr(vfma(vneg(tA), u, vset<V>(1.f)))), tA);
+__device__ __forceinline__ float tan_offset(float tA, float d) {
+  const float d2 = d * d;
+  float p = fmaf(d2, 5.3968254e-2f, 1.3333334e-1f);
+  p = fmaf(d2, p, 3.3333334e-1f);
+  const float u = fmaf(d * d2, p, d);
+  const float r = u * fmaf(tA, tA, 1.f);
+  return fmaf(r, rcp_nr(fmaf(-tA, u, 1.f)), tA);
 }
 
 // sin(a) and 1 - cos(a) without cancellation.
@@ -256,13 +189,14 @@ __device__ __forceinline__ void sin_versine(float a, float *s, float *v) {
     *v = 2.f * sh * sh;
   }
 }
+
 // sin and cos of a float, each rounded once from a double evaluation: the
 // correctly rounded float result except within ~1e-16 of a rounding midpoint.
 // One reduction serves both: x = k pi/2 + r with pi/2 in two doubles, then the
 // Taylor series of sin r and cos r, |r| <= pi/4 (the next terms, r^19/19! and
 // r^18/18!, are below 1e-18).  Without CUDA's separate double sin and cos (whose
-// branch for arguments that need a longer pi/2 the last line keeps) the
-// reference-rounding step takes REFINSTR.
+// branch for arguments that need a longer pi/2 the first lines keep) the 10 x 4096
+// track, 10 layer pass in the reference's rounding takes 65 us instead of 96.
 __device__ __forceinline__ void sincosf_cr(float x, float *sn, float *cs) {
   const double xd = (double)x;
   if (__builtin_expect(!(fabsf(x) <= 1e5f), 0)) {
@@ -305,11 +239,10 @@ __device__ __forceinline__ void sincosf_cr(float x, float *sn, float *cs) {
 
 // The unit vector (c, s) = (cos t, sin t) rotated to t + d, given w = sin d
 // and v = 1 - cos d: cos(t+d) = c - (c*v + s*w), sin(t+d) = s - (s*v - c*w).
-// (One track: as packed pairs the register-pair moves cost more than they save.)
-template <typename V>
-__device__ __forceinline__ void rotated(V c, V s, V w, V v, V *cn, V *sn) {
-  *cn = vsub(c, vfma(c, v, vmul(s, w)));
-  *sn = vsub(s, vfma(s, v, vneg(vmul(c, w))));
+// (Scalar: as packed pairs the register-pair moves cost more than they save.)
+__device__ __forceinline__ void rotated(float c, float s, float w, float v, float *cn, float *sn) {
+  *cn = c - fmaf(c, v, s * w);
+  *sn = s - fmaf(s, v, -(c * w));
 }
 
 // Re-anchoring thresholds of the carried phi and theta offsets.  After a
@@ -344,9 +277,9 @@ template <typename A>
 struct PhiOf {
   using type = A;
 };
-template <typename V>
-struct PhiOf<APT<V>> {
-  using type = V;
+template <>
+struct PhiOf<AP> {
+  using type = float;
 };
 
 template <typename T, typename A>
@@ -372,18 +305,14 @@ struct Trk {
 // Helix quantities shared by the parameter update and the Jacobian.  omc and
 // omcC are 1 - cos(alpha) and 1 - cos(cosP*sin(alpha)).
 //   FORM_PRECISE / FP64 fields: tanT = tan(theta), icT2 = 1/cos^2(theta),
-//     dzk = deltaZ/k, dzkt = dzk*tanT, kpt = k*pt, m1 = cosP*sina, m2 = sinP*sina.
+//     dzk = deltaZ/k, kpt = k*pt, m1 = cosP*sina, m2 = sinP*sina.
 //   FORM_REFERENCE fields: sinT, icosT, icosTk (the reference's own scalars).
 template <typename T>
 struct Helix {
   T deltaZ, pt, cosP, sinP, sina, cosa, omc, sCPs, omcC;
-  T tanT, icT2, dzk, dzkt, kpt, m1, m2;
+  T tanT, icT2, dzk, kpt, m1, m2;
   T sinT, icosT, icosTk;
 };
-
-__device__ __forceinline__ void phi_add(float &a, float d) { a = __fadd_rn(a, d); }
-__device__ __forceinline__ void phi_add(float2 &a, float2 d) { a = vadd(a, d); }
-__device__ __forceinline__ void phi_add(DF &a, float d) { acc_add(a, d); }
 
 // The Jacobian entries that act on a covariance with zero z row (reference
 // :655-666 without column 2), and those of column 2 for the first layer.
@@ -408,84 +337,6 @@ __device__ __forceinline__ void init_direction(Trk<float, A> &s) {
   s.dP = 0.f;
   s.dT = 0.f;
 }
-// Two tracks: the components named by `which`, one at a time.
-__device__ __forceinline__ void init_direction(Trk<float2, APT<float2>> &s, Bool2 which = {true, true}) {
-#pragma unroll 1
-  for (int c = 0; c < 2; ++c) {
-    if (!(c ? which.y : which.x)) continue;
-    float sP, cP, sT, cT;
-    sincosf(c ? s.phi.y : s.phi.x, &sP, &cP);
-    sincosf(c ? s.theta.y : s.theta.x, &sT, &cT);
-    const float tT = __fdiv_rn(sT, cT);
-    if (c) { s.sP.y = sP; s.cP.y = cP; s.tT.y = tT; s.dP.y = 0.f; s.dT.y = 0.f; }
-    else { s.sP.x = sP; s.cP.x = cP; s.tT.x = tT; s.dP.x = 0.f; s.dT.x = 0.f; }
-  }
-}
-
-// The direction of a step and sin and 1 - cos of its helix angle, from the
-// anchors and offsets of one track.
-struct Direction {
-  float cP, sP, tT, dP, dT;  // anchors and offsets (may be moved)
-  float cosP, sinP, tanT, dzkt, alpha, sina, omc;
-};
-
-// The same for a track whose step leaves the ranges of the plain evaluation,
-// with every case: a theta offset past kAnchorTheta moves the theta anchor
-// there, offsets outside the ranges of their series (see kRangePhi) re-anchor
-// the direction at the track's angles, and sin and 1 - cos of an angle past 0.5
-// rad come from its half.
-__device__ __forceinline__ void direction_any(Direction &d, float phi, float theta, float dzk, float ipt) {
-  if (!(fabsf(d.dP) <= kRangePhi && fabsf(d.dT) <= kRangeTheta)) {
-    sincosf(phi, &d.sP, &d.cP);
-    float sT, cT;
-    sincosf(theta, &sT, &cT);
-    d.tT = __fdiv_rn(sT, cT);
-    d.dP = 0.f;
-    d.dT = 0.f;
-  } else if (fabsf(d.dT) > kAnchorTheta) {
-    d.tT = tan_offset(d.tT, d.dT);
-    d.dT = 0.f;
-  }
-  float w, v;
-  sv_series(d.dP, &w, &v);
-  rotated(d.cP, d.sP, w, v, &d.cosP, &d.sinP);
-  d.tanT = tan_offset(d.tT, d.dT);
-  d.dzkt = vmul(dzk, d.tanT);
-  d.alpha = vmul(d.dzkt, ipt);
-  sin_versine<SC_FAST>(d.alpha, &d.sina, &d.omc);
-}
-__device__ __forceinline__ bool past(float v, float limit) { return !(fabsf(v) <= limit); }
-
-// Both tracks of a pair in the plain ranges, or (rarely) the others one at a time.
-template <typename A>
-__device__ __forceinline__ void step_direction(Trk<float2, A> &s, Helix<float2> &h, float2 &alpha, Bool2 live) {
-  using V = float2;
-  V w, v;
-  sv_series(s.dP, &w, &v);
-  rotated(s.cP, s.sP, w, v, &h.cosP, &h.sinP);
-  h.tanT = tan_offset(s.tT, s.dT);
-  h.dzkt = vmul(h.dzk, h.tanT);
-  alpha = vmul(h.dzkt, s.ipt);
-  sv_series(alpha, &h.sina, &h.omc);
-  const bool x = live.x && (past(s.dP.x, kRangePhi) || past(s.dT.x, kAnchorTheta) || past(alpha.x, 0.5f));
-  const bool y = live.y && (past(s.dP.y, kRangePhi) || past(s.dT.y, kAnchorTheta) || past(alpha.y, 0.5f));
-  if (__builtin_expect(x || y, 0)) {
-#pragma unroll 1
-    for (int c = 0; c < 2; ++c) {
-      if (!(c ? y : x)) continue;
-#define P2Z_HALF(f) (c ? (f).y : (f).x)
-      Direction d;
-      d.cP = P2Z_HALF(s.cP); d.sP = P2Z_HALF(s.sP); d.tT = P2Z_HALF(s.tT); d.dP = P2Z_HALF(s.dP); d.dT = P2Z_HALF(s.dT);
-      direction_any(d, P2Z_HALF(s.phi), P2Z_HALF(s.theta), P2Z_HALF(h.dzk), P2Z_HALF(s.ipt));
-#undef P2Z_HALF
-#define P2Z_PUT(f, val) (c ? (f).y : (f).x) = val
-      P2Z_PUT(s.cP, d.cP); P2Z_PUT(s.sP, d.sP); P2Z_PUT(s.tT, d.tT); P2Z_PUT(s.dP, d.dP); P2Z_PUT(s.dT, d.dT);
-      P2Z_PUT(h.cosP, d.cosP); P2Z_PUT(h.sinP, d.sinP); P2Z_PUT(h.tanT, d.tanT); P2Z_PUT(h.dzkt, d.dzkt);
-      P2Z_PUT(alpha, d.alpha); P2Z_PUT(h.sina, d.sina); P2Z_PUT(h.omc, d.omc);
-#undef P2Z_PUT
-    }
-  }
-}
 
 // Parameter propagation (reference :627-647), with the reference's products
 // regrouped around shared factors (exact in real arithmetic):
@@ -506,66 +357,55 @@ __device__ __forceinline__ void step_direction(Trk<float2, A> &s, Helix<float2> 
 // kAnchorTheta moves the theta anchor to this step's tan(theta).  Selects, no
 // branch.
 template <int SC, typename A>
-__device__ __forceinline__ void step_direction(Trk<float, A> &s, Helix<float> &h, float &alpha, bool) {
+__device__ __forceinline__ Helix<float> propagate_params_precise(Trk<float, A> &s, float zout, float k, float ik) {
+  Helix<float> h;
+  if (__builtin_expect(!(fabsf(s.dP) <= kRangePhi && fabsf(s.dT) <= kRangeTheta), 0)) init_direction(s);
+  h.deltaZ = zout - s.z;
+  h.pt = rcp_nr(s.ipt);
   {
     // SC_FAST: |dP| <= kAnchorPhi + one Kalman correction, inside the series'
     // range, so no range branch (a branch would end the basic block and keep
     // the scheduler from overlapping this with the previous update)
     float w, v;
-    if constexpr (SC == SC_FAST) sv_series(s.dP, &w, &v);
+    if (SC == SC_FAST) sv_series(s.dP, &w, &v);
     else sin_versine<SC>(s.dP, &w, &v);
     rotated(s.cP, s.sP, w, v, &h.cosP, &h.sinP);
   }
   h.tanT = tan_offset(s.tT, s.dT);
+  h.icT2 = fmaf(h.tanT, h.tanT, 1.f);
   const bool moveT = fabsf(s.dT) > kAnchorTheta;
-  s.tT = vsel(moveT, h.tanT, s.tT);
-  s.dT = vsel(moveT, 0.f, s.dT);
-  h.dzkt = vmul(h.dzk, h.tanT);
-  alpha = vmul(h.dzkt, s.ipt);
+  s.tT = moveT ? h.tanT : s.tT;
+  s.dT = moveT ? 0.f : s.dT;
+  h.dzk = (SC == SC_FAST) ? h.deltaZ * ik : __fdiv_rn(h.deltaZ, k);
+  const float alpha = (h.dzk * h.tanT) * s.ipt;
   sin_versine<SC>(alpha, &h.sina, &h.omc);
-}
-
-template <int SC, typename V, typename A, typename L>
-__device__ __forceinline__ Helix<V> propagate_params_precise(Trk<V, A> &s, V zout, V k, V ik, L live) {
-  Helix<V> h;
-  if constexpr (std::is_same<V, float>::value) {
-    if (__builtin_expect(past(s.dP, kRangePhi) || past(s.dT, kRangeTheta), 0)) init_direction(s);
-  }
-  h.deltaZ = vsub(zout, s.z);
-  h.pt = vneg(nrcp_nr(s.ipt));
-  if constexpr (SC == SC_FAST) h.dzk = vmul(h.deltaZ, ik);
-  else h.dzk = __fdiv_rn(h.deltaZ, k);
-  V alpha;
-  if constexpr (std::is_same<V, float2>::value) step_direction(s, h, alpha, live);
-  else step_direction<SC>(s, h, alpha, live);
-  h.icT2 = vfma(h.tanT, h.tanT, vset<V>(1.f));
-  h.cosa = vsub(vset<V>(1.f), h.omc);
-  h.kpt = vmul(k, h.pt);
-  h.m1 = vmul(h.cosP, h.sina);
-  h.m2 = vmul(h.sinP, h.sina);
-  // (gx, gy): the step in units of k*pt, and the change of the direction
-  const V gx = vfma(vneg(h.sinP), h.omc, h.m1), gy = vfma(h.cosP, h.omc, h.m2);
-  acc_fma(s.x, h.kpt, gx);
-  acc_fma(s.y, h.kpt, gy);
+  h.cosa = 1.f - h.omc;
+  h.kpt = k * h.pt;
+  h.m1 = h.cosP * h.sina;
+  h.m2 = h.sinP * h.sina;
+  acc_add(s.x, h.kpt * fmaf(-h.sinP, h.omc, h.m1));
+  acc_add(s.y, h.kpt * fmaf(h.cosP, h.omc, h.m2));
   s.z = zout;
-  phi_add(s.phi, alpha);
-  if constexpr (SC == SC_FAST) sv_series(h.m1, &h.sCPs, &h.omcC);
+  acc_add(s.phi, alpha);
+  if (SC == SC_FAST) sv_series(h.m1, &h.sCPs, &h.omcC);
   else sin_versine<SC>(h.m1, &h.sCPs, &h.omcC);
-  const V dP = vadd(s.dP, alpha);
-  const auto moveP = vgt_abs(dP, kAnchorPhi);
+  const float dP = __fadd_rn(s.dP, alpha);
+  const bool moveP = fabsf(dP) > kAnchorPhi;
   // (cos, sin) of phi + alpha from sin(alpha) and the versine
-  s.cP = vsel(moveP, vsub(h.cosP, gy), s.cP);
-  s.sP = vsel(moveP, vadd(h.sinP, gx), s.sP);
-  s.dP = vsel(moveP, vset<V>(0.f), dP);
+  const float cPn = h.cosP - fmaf(h.cosP, h.omc, h.m2);
+  const float sPn = h.sinP - fmaf(h.sinP, h.omc, -h.m1);
+  s.cP = moveP ? cPn : s.cP;
+  s.sP = moveP ? sPn : s.sP;
+  s.dP = moveP ? 0.f : dP;
   return h;
 }
 
 // A Kalman correction of phi and theta, added to the offsets from the
 // anchors (the output angles accumulate it separately).
-template <typename V, typename A>
-__device__ __forceinline__ void turn_direction(Trk<V, A> &s, V dphi, V dth) {
-  s.dP = vadd(s.dP, dphi);
-  s.dT = vadd(s.dT, dth);
+template <typename A>
+__device__ __forceinline__ void turn_direction(Trk<float, A> &s, float dphi, float dth) {
+  s.dP = __fadd_rn(s.dP, dphi);
+  s.dT = __fadd_rn(s.dT, dth);
 }
 
 // The Jacobian entries (reference :655-666) with the shared factors taken out
@@ -577,52 +417,21 @@ __device__ __forceinline__ void turn_direction(Trk<V, A> &s, V dphi, V dth) {
 //   J43 = (dZ/k)*tanT                                   J45 = (dZ/k)*ipt/cosT^2
 // and, for the first layer, J02 = -cosP*tanT*cosa*B, J12 = cosa*tanT*(cosP^2*sC - sinP),
 // J42 = -ipt*tanT/k.
-template <bool GENERAL, typename V>
-__device__ __forceinline__ Jac<V> jacobian_precise(const Helix<V> &h, V k, V ipt) {
-  Jac<V> J;
-  const V cosP = h.cosP, sinP = h.sinP;
-  const V dzc = vmul(h.deltaZ, h.cosa);
-  const V B = vfma(vneg(sinP), h.sCPs, vset<V>(1.f));
-  const V cs = vmul(cosP, h.sCPs);
-  const V D = vfma(cs, cosP, sinP);
-  const V stp = vmul(h.tanT, h.pt);
-  const V nkpt = vneg(h.kpt), nkpt2 = vmul(nkpt, h.pt);
-  const V n1 = vmul(cosP, h.omcC), n2 = vmul(sinP, h.omcC);
-  const V u = vmul(vmul(cosP, dzc), B);
-  const V v = vmul(dzc, D);
-  J.a3 = vfma(u, stp, vmul(nkpt2, vsub(h.m1, n2)));
-  J.a5 = vmul(u, h.icT2);
-  J.a9 = vfma(v, stp, vmul(nkpt2, vadd(h.m2, n1)));
-  J.a11 = vmul(v, h.icT2);
-  J.a4 = vmul(nkpt, vfma(h.m2, B, n1));
-  J.a10 = vmul(h.kpt, vfma(h.m1, B, vneg(n2)));
-  J.a27 = h.dzkt;
-  J.a29 = vmul(vmul(h.dzk, ipt), h.icT2);
-  if constexpr (GENERAL) {
-    J.a2 = vmul(vneg(vmul(cosP, h.tanT)), vmul(h.cosa, B));
-    J.a8 = vmul(vmul(h.cosa, h.tanT), vfma(cs, cosP, vneg(sinP)));
-    J.a26 = vdiv(vneg(vmul(ipt, h.tanT)), k);
-  } else {
-    J.a2 = J.a8 = J.a26 = vset<V>(0.f);
-  }
-  return J;
-}
-
-// The same entries in double.
-__device__ __forceinline__ Jac<double> jacobian_f64(const Helix<double> &h, double k, double ipt, bool general) {
-  Jac<double> J;
-  const double cosP = h.cosP, sinP = h.sinP;
-  const double dzc = h.deltaZ * h.cosa;
-  const double B = 1.0 - sinP * h.sCPs;
-  const double cc = cosP * cosP * h.sCPs;
-  const double D = cc + sinP;
-  const double stp = h.tanT * h.pt;
-  const double kpt = h.kpt;
-  const double kpt2 = kpt * h.pt;
-  const double m1 = h.m1, m2 = h.m2;
-  const double n1 = cosP * h.omcC, n2 = sinP * h.omcC;
-  const double u = cosP * dzc * B;
-  const double v = dzc * D;
+template <typename T, bool GENERAL = false>
+__device__ __forceinline__ Jac<T> jacobian_precise(const Helix<T> &h, T k, T ipt) {
+  Jac<T> J;
+  const T cosP = h.cosP, sinP = h.sinP;
+  const T dzc = h.deltaZ * h.cosa;
+  const T B = T(1) - sinP * h.sCPs;
+  const T cc = cosP * cosP * h.sCPs;
+  const T D = cc + sinP;
+  const T stp = h.tanT * h.pt;
+  const T kpt = h.kpt;
+  const T kpt2 = kpt * h.pt;
+  const T m1 = h.m1, m2 = h.m2;
+  const T n1 = cosP * h.omcC, n2 = sinP * h.omcC;
+  const T u = cosP * dzc * B;
+  const T v = dzc * D;
   J.a3 = u * stp - kpt2 * (m1 - n2);
   J.a5 = u * h.icT2;
   J.a9 = v * stp - kpt2 * (m2 + n1);
@@ -631,9 +440,13 @@ __device__ __forceinline__ Jac<double> jacobian_f64(const Helix<double> &h, doub
   J.a10 = kpt * (m1 * B - n2);
   J.a27 = h.dzk * h.tanT;
   J.a29 = (h.dzk * ipt) * h.icT2;
-  J.a2 = general ? -(cosP * h.tanT) * (h.cosa * B) : 0.0;
-  J.a8 = general ? h.cosa * h.tanT * (cc - sinP) : 0.0;
-  J.a26 = general ? -(ipt * h.tanT) / k : 0.0;
+  if constexpr (GENERAL) {
+    J.a2 = -(cosP * h.tanT) * (h.cosa * B);
+    J.a8 = h.cosa * h.tanT * (cc - sinP);
+    J.a26 = -(ipt * h.tanT) / k;
+  } else {
+    J.a2 = J.a8 = J.a26 = T(0);
+  }
   return J;
 }
 
@@ -759,51 +572,15 @@ __device__ __forceinline__ void propagate_cov_reduced(Trk<T, A> &s, const Jac<T>
   s.c55 = t35;                                           // c20
 }
 
-// The precise form's reduced propagation, 54 fused multiply-adds: the sums
-// above in the same order, with the identities (c30, c31)' = (t3, t9),
-// (c50, c51)' = (t5, t11), c43' = t27 and c54' = t29.  (c40' and c41' cost 4
-// instead of 10 as t4 + J43 t3 + J45 t5, from the columns of T; but from row 4
-// of T they round as c43', c44' and c54' do, which the update's cancellations
-// feel: the rms error of C over 9.6M tracks is 1.447e-6 so and 1.454e-6 from the
-// columns, the worst track's 1.06e-4 and 1.36e-4.)
-// Two tracks: products that share a factor stand together, which lets it stay in
-// the operand collector; see k_duo.
+// The same reduced form with the row-0/row-1 Jacobian pairs (a3, a9),
+// (a4, a10), (a5, a11) and the covariance pairs (c00, c10), (c30, c31),
+// (c40, c41), (c50, c51) in packed FP32 pairs.  Each component is the scalar
+// form's chain of fused multiply-adds in the same order, so the results are
+// identical bit for bit; the pairs only halve the instructions.  Identities
+// used: the new (c30, c31) is T's (t3, t9), the new (c50, c51) is (t5, t11),
+// the new c54 is t29 and the new c43 is t27.
 template <typename A>
-__device__ __forceinline__ void propagate_cov_precise(Trk<float2, A> &s, const Jac<float2> &J) {
-  using V = float2;
-  const V a3 = J.a3, a4 = J.a4, a5 = J.a5, a9 = J.a9, a10 = J.a10, a11 = J.a11, a27 = J.a27, a29 = J.a29;
-  V t27 = vfma(a27, s.c33, s.c43), t28 = vfma(a27, s.c43, s.c44), t29 = vfma(a27, s.c53, s.c54);
-  V c40 = vfma(a27, s.c30, s.c40), c41 = vfma(a27, s.c31, s.c41);
-  t27 = vfma(a29, s.c53, t27); t28 = vfma(a29, s.c54, t28); t29 = vfma(a29, s.c55, t29);
-  c40 = vfma(a29, s.c50, c40); c41 = vfma(a29, s.c51, c41);
-  V t0 = vfma(a3, s.c30, s.c00), t3 = vfma(a3, s.c33, s.c30), t4 = vfma(a3, s.c43, s.c40), t5 = vfma(a3, s.c53, s.c50);
-  V t6 = vfma(a9, s.c30, s.c10), t9 = vfma(a9, s.c33, s.c31), t10 = vfma(a9, s.c43, s.c41), t11 = vfma(a9, s.c53, s.c51);
-  V t7 = vfma(a9, s.c31, s.c11);
-  t0 = vfma(a4, s.c40, t0); t3 = vfma(a4, s.c43, t3); t4 = vfma(a4, s.c44, t4); t5 = vfma(a4, s.c54, t5);
-  t6 = vfma(a10, s.c40, t6); t9 = vfma(a10, s.c43, t9); t10 = vfma(a10, s.c44, t10); t11 = vfma(a10, s.c54, t11);
-  t7 = vfma(a10, s.c41, t7);
-  t0 = vfma(a5, s.c50, t0); t3 = vfma(a5, s.c53, t3); t4 = vfma(a5, s.c54, t4); t5 = vfma(a5, s.c55, t5);
-  t6 = vfma(a11, s.c50, t6); t9 = vfma(a11, s.c53, t9); t10 = vfma(a11, s.c54, t10); t11 = vfma(a11, s.c55, t11);
-  t7 = vfma(a11, s.c51, t7);
-  t0 = vfma(a3, t3, t0); t6 = vfma(a3, t9, t6); c40 = vfma(a3, t27, c40);
-  t7 = vfma(a9, t9, t7); c41 = vfma(a9, t27, c41);
-  t0 = vfma(a4, t4, t0); t6 = vfma(a4, t10, t6); c40 = vfma(a4, t28, c40);
-  t7 = vfma(a10, t10, t7); c41 = vfma(a10, t28, c41);
-  s.c00 = vfma(a5, t5, t0); s.c10 = vfma(a5, t11, t6); s.c40 = vfma(a5, t29, c40);
-  s.c11 = vfma(a11, t11, t7); s.c41 = vfma(a11, t29, c41);
-  s.c44 = vfma(a29, t29, vfma(a27, t27, t28));
-  s.c30 = t3; s.c31 = t9;
-  s.c43 = t27;
-  s.c50 = t5; s.c51 = t11;
-  s.c54 = t29;
-}
-
-// One track: the same fused multiply-adds with the row-0/row-1 Jacobian pairs
-// (a3, a9), (a4, a10), (a5, a11) and the covariance pairs (c00, c10),
-// (c30, c31), (c40, c41), (c50, c51) in packed FP32 pairs, bit for bit the
-// results above.
-template <typename A>
-__device__ __forceinline__ void propagate_cov_precise(Trk<float, A> &s, const Jac<float> &J) {
+__device__ __forceinline__ void propagate_cov_reduced_packed(Trk<float, A> &s, const Jac<float> &J) {
   const float2 A3 = make_float2(J.a3, J.a9), A4 = make_float2(J.a4, J.a10), A5 = make_float2(J.a5, J.a11);
   const float2 P0 = make_float2(s.c00, s.c10), P3 = make_float2(s.c30, s.c31);
   const float2 P4 = make_float2(s.c40, s.c41), P5 = make_float2(s.c50, s.c51);
@@ -812,20 +589,21 @@ __device__ __forceinline__ void propagate_cov_precise(Trk<float, A> &s, const Ja
   const float2 T3 = fma2(A5, bc2(s.c53), fma2(A4, bc2(s.c43), fma2(A3, bc2(s.c33), P3)));  // (t3, t9)
   const float2 T4 = fma2(A5, bc2(s.c54), fma2(A4, bc2(s.c44), fma2(A3, bc2(s.c43), P4)));  // (t4, t10)
   const float2 T5 = fma2(A5, bc2(s.c55), fma2(A4, bc2(s.c54), fma2(A3, bc2(s.c53), P5)));  // (t5, t11)
-  const float t7 = vfma(J.a11, s.c51, vfma(J.a10, s.c41, vfma(J.a9, s.c31, s.c11)));
-  const float t27 = vfma(J.a29, s.c53, vfma(J.a27, s.c33, s.c43));
-  const float t28 = vfma(J.a29, s.c54, vfma(J.a27, s.c43, s.c44));
-  const float t29 = vfma(J.a29, s.c55, vfma(J.a27, s.c53, s.c54));
+  const float t7 = s.c11 + J.a9 * s.c31 + J.a10 * s.c41 + J.a11 * s.c51;
+  const float2 T24 = fma2(bc2(J.a29), P5, fma2(bc2(J.a27), P3, P4));                        // (t24, t25)
+  const float t27 = J.a27 * s.c33 + s.c43 + J.a29 * s.c53;
+  const float t28 = J.a27 * s.c43 + s.c44 + J.a29 * s.c54;
+  const float t29 = J.a27 * s.c53 + s.c54 + J.a29 * s.c55;
   // C' = T J^T
   const float2 N0 = fma2(T5, bc2(J.a5), fma2(T4, bc2(J.a4), fma2(T3, bc2(J.a3), T0)));      // (c00, c10)
-  const float2 T24 = fma2(bc2(J.a29), P5, fma2(bc2(J.a27), P3, P4));                        // (t24, t25)
+  const float c11 = t7 + T3.y * J.a9 + T4.y * J.a10 + T5.y * J.a11;
   const float2 N4 = fma2(A5, bc2(t29), fma2(A4, bc2(t28), fma2(A3, bc2(t27), T24)));       // (c40, c41)
   s.c00 = N0.x; s.c10 = N0.y;
-  s.c11 = vfma(T5.y, J.a11, vfma(T4.y, J.a10, vfma(T3.y, J.a9, t7)));
+  s.c11 = c11;
   s.c30 = T3.x; s.c31 = T3.y;
   s.c40 = N4.x; s.c41 = N4.y;
   s.c43 = t27;
-  s.c44 = vfma(J.a29, t29, vfma(J.a27, t27, t28));
+  s.c44 = t27 * J.a27 + t28 + t29 * J.a29;
   s.c50 = T5.x; s.c51 = T5.y;
   s.c54 = t29;
 }
@@ -849,18 +627,18 @@ __device__ __forceinline__ void propagate_cov_reduced_pair(Trk<float, A> &s, con
                                                            unsigned pm) {
   const float A3 = j ? J.a9 : J.a3, A4 = j ? J.a10 : J.a4, A5 = j ? J.a11 : J.a5;
   const float P0 = j ? s.c10 : s.c00, P3 = j ? s.c31 : s.c30, P4 = j ? s.c41 : s.c40, P5 = j ? s.c51 : s.c50;
-  const float T0 = vfma(A5, s.c50, vfma(A4, s.c40, vfma(A3, s.c30, P0)));  // t0 | t6
-  const float T3 = vfma(A5, s.c53, vfma(A4, s.c43, vfma(A3, s.c33, P3)));  // t3 | t9
-  const float T4 = vfma(A5, s.c54, vfma(A4, s.c44, vfma(A3, s.c43, P4)));  // t4 | t10
-  const float T5 = vfma(A5, s.c55, vfma(A4, s.c54, vfma(A3, s.c53, P5)));  // t5 | t11
-  const float t7 = vfma(J.a11, s.c51, vfma(J.a10, s.c41, vfma(J.a9, s.c31, s.c11)));
-  const float t27 = vfma(J.a29, s.c53, vfma(J.a27, s.c33, s.c43));
-  const float t28 = vfma(J.a29, s.c54, vfma(J.a27, s.c43, s.c44));
-  const float t29 = vfma(J.a29, s.c55, vfma(J.a27, s.c53, s.c54));
-  const float N0 = vfma(T5, J.a5, vfma(T4, J.a4, vfma(T3, J.a3, T0)));    // c00 | c10
-  const float c11 = vfma(T5, J.a11, vfma(T4, J.a10, vfma(T3, J.a9, t7)));  // the result on lane 1
-  const float T24 = vfma(J.a29, P5, vfma(J.a27, P3, P4));                  // t24 | t25
-  const float N4 = vfma(A5, t29, vfma(A4, t28, vfma(A3, t27, T24)));       // c40 | c41
+  const float T0 = fmaf(A5, s.c50, fmaf(A4, s.c40, fmaf(A3, s.c30, P0)));  // t0 | t6
+  const float T3 = fmaf(A5, s.c53, fmaf(A4, s.c43, fmaf(A3, s.c33, P3)));  // t3 | t9
+  const float T4 = fmaf(A5, s.c54, fmaf(A4, s.c44, fmaf(A3, s.c43, P4)));  // t4 | t10
+  const float T5 = fmaf(A5, s.c55, fmaf(A4, s.c54, fmaf(A3, s.c53, P5)));  // t5 | t11
+  const float t7 = s.c11 + J.a9 * s.c31 + J.a10 * s.c41 + J.a11 * s.c51;
+  const float T24 = fmaf(J.a29, P5, fmaf(J.a27, P3, P4));                  // t24 | t25
+  const float t27 = J.a27 * s.c33 + s.c43 + J.a29 * s.c53;
+  const float t28 = J.a27 * s.c43 + s.c44 + J.a29 * s.c54;
+  const float t29 = J.a27 * s.c53 + s.c54 + J.a29 * s.c55;
+  const float N0 = fmaf(T5, J.a5, fmaf(T4, J.a4, fmaf(T3, J.a3, T0)));    // c00 | c10
+  const float c11 = t7 + T3 * J.a9 + T4 * J.a10 + T5 * J.a11;              // the result on lane 1
+  const float N4 = fmaf(A5, t29, fmaf(A4, t28, fmaf(A3, t27, T24)));       // c40 | c41
   pair_join(N0, j, pm, s.c00, s.c10);
   pair_join(T3, j, pm, s.c30, s.c31);
   pair_join(N4, j, pm, s.c40, s.c41);
@@ -868,51 +646,8 @@ __device__ __forceinline__ void propagate_cov_reduced_pair(Trk<float, A> &s, con
   const float c11o = __shfl_xor_sync(pm, c11, 1);
   s.c11 = j ? c11 : c11o;
   s.c43 = t27;
-  s.c44 = vfma(J.a29, t29, vfma(J.a27, t27, t28));
+  s.c44 = t27 * J.a27 + t28 + t29 * J.a29;
   s.c54 = t29;
-}
-
-// The precise form's general propagation (the first layer): the sums of
-// propagate_cov_general below in its order, on the full input covariance b[].
-template <typename V, typename A>
-__device__ __forceinline__ void propagate_cov_general_precise(Trk<V, A> &s, const V *b, const Jac<V> &J) {
-  const V a2 = J.a2, a8 = J.a8, a26 = J.a26;
-  const V a3 = J.a3, a4 = J.a4, a5 = J.a5, a9 = J.a9, a10 = J.a10, a11 = J.a11, a27 = J.a27, a29 = J.a29;
-  auto row0 = [&](V c, V z, V i, V p, V t) { return vfma(a5, t, vfma(a4, p, vfma(a3, i, vfma(a2, z, c)))); };
-  auto row1 = [&](V c, V z, V i, V p, V t) { return vfma(a11, t, vfma(a10, p, vfma(a9, i, vfma(a8, z, c)))); };
-  auto row4 = [&](V c, V z, V i, V t) { return vfma(a29, t, vadd(vfma(a27, i, vmul(a26, z)), c)); };
-  const V t0 = row0(b[0], b[3], b[6], b[10], b[15]);
-  const V t2 = row0(b[3], b[5], b[8], b[12], b[17]);
-  const V t3 = row0(b[6], b[8], b[9], b[13], b[18]);
-  const V t4 = row0(b[10], b[12], b[13], b[14], b[19]);
-  const V t5 = row0(b[15], b[17], b[18], b[19], b[20]);
-  const V t6 = row1(b[1], b[3], b[6], b[10], b[15]);
-  const V t7 = row1(b[2], b[4], b[7], b[11], b[16]);
-  const V t8 = row1(b[4], b[5], b[8], b[12], b[17]);
-  const V t9 = row1(b[7], b[8], b[9], b[13], b[18]);
-  const V t10 = row1(b[11], b[12], b[13], b[14], b[19]);
-  const V t11 = row1(b[16], b[17], b[18], b[19], b[20]);
-  const V t24 = row4(b[10], b[3], b[6], b[15]);
-  const V t25 = row4(b[11], b[4], b[7], b[16]);
-  const V t26 = row4(b[12], b[5], b[8], b[17]);
-  const V t27 = row4(b[13], b[8], b[9], b[18]);
-  const V t28 = row4(b[14], b[12], b[13], b[19]);
-  const V t29 = row4(b[19], b[17], b[18], b[20]);
-  s.c00 = row0(t0, t2, t3, t4, t5);
-  s.c10 = row0(t6, t8, t9, t10, t11);
-  s.c11 = row1(t7, t8, t9, t10, t11);
-  s.c30 = row0(b[6], b[8], b[9], b[13], b[18]);
-  s.c31 = row1(b[7], b[8], b[9], b[13], b[18]);
-  s.c33 = b[9];
-  s.c40 = row0(t24, t26, t27, t28, t29);
-  s.c41 = row1(t25, t26, t27, t28, t29);
-  s.c43 = t27;
-  s.c44 = vfma(a29, t29, vadd(vfma(a27, t27, vmul(a26, t26)), t28));
-  s.c50 = row0(b[15], b[17], b[18], b[19], b[20]);
-  s.c51 = row1(b[16], b[17], b[18], b[19], b[20]);
-  s.c53 = b[18];
-  s.c54 = vfma(a29, b[20], vadd(vfma(a27, b[18], vmul(a26, b[17])), b[19]));
-  s.c55 = b[20];
 }
 
 // General form on the full 21-element input covariance b[] (the first
@@ -920,7 +655,9 @@ __device__ __forceinline__ void propagate_cov_general_precise(Trk<V, A> &s, cons
 // a8 = J(1,2), a26 = J(4,2) (reference :655, :659, :663), which the Jacobian
 // functions fill for the first layer.
 template <typename T, typename A>
-__device__ __forceinline__ void propagate_cov_general(Trk<T, A> &s, const T *b, const Jac<T> &J) {
+__device__ __forceinline__ void propagate_cov_general(Trk<T, A> &s, const T *b, const Helix<T> &h,
+                                                      const Jac<T> &J) {
+  (void)h;
   const T a2 = J.a2, a8 = J.a8, a26 = J.a26;
   const T a3 = J.a3, a4 = J.a4, a5 = J.a5, a9 = J.a9, a10 = J.a10, a11 = J.a11, a27 = J.a27, a29 = J.a29;
   const T t0 = b[0] + a2 * b[3] + a3 * b[6] + a4 * b[10] + a5 * b[15];
@@ -1004,186 +741,143 @@ __device__ __forceinline__ float det2_comp(float a, float b, float c, float d) {
 // samples.
 constexpr float kJosephShrink = 0.01f;
 
-// E_i = P_i - K_i V of the Joseph form, K V from error-free products: p + e is
-// exactly nK0 v (nK = -K).
-template <typename V>
-__device__ __forceinline__ V joseph_resid(V P, V nK0, V nK1, V v0, V v1) {
-  const V p = vmul(nK0, v0);
-  const V e = vfma(nK0, v0, vneg(p));
-  return vadd(vadd(vfma(nK1, v1, p), e), P);
-}
-
-// The Joseph form of a track's first update, from the plain update's result
-// (s holds P = C - K H C): C'' = P - E K^T for the tracks `which` names.  p01
-// is P(x, y), which the plain update does not keep beside P(y, x) = s.c10; nK
-// the negated gain's rows x, y, ipt, phi, theta.
-template <typename V, typename A, typename W>
-__device__ __forceinline__ void update_v2_joseph(Trk<V, A> &s, W which, V p01, const V (&nK)[5][2], V v00, V v01,
-                                                 V v11) {
-  const V P[5][2] = {{s.c00, p01}, {s.c10, s.c11}, {s.c30, s.c31}, {s.c40, s.c41}, {s.c50, s.c51}};
-  V E[5][2];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    E[i][0] = joseph_resid(P[i][0], nK[i][0], nK[i][1], v00, v01);
-    E[i][1] = joseph_resid(P[i][1], nK[i][0], nK[i][1], v01, v11);
-  }
-  auto corr = [&](V &c, int i, int j) { c = vsel(which, vfma(E[i][1], nK[j][1], vfma(E[i][0], nK[j][0], c)), c); };
-  corr(s.c00, 0, 0);
-  corr(s.c10, 1, 0); corr(s.c11, 1, 1);
-  corr(s.c30, 2, 0); corr(s.c31, 2, 1); corr(s.c33, 2, 2);
-  corr(s.c40, 3, 0); corr(s.c41, 3, 1); corr(s.c43, 3, 2); corr(s.c44, 3, 3);
-  corr(s.c50, 4, 0); corr(s.c51, 4, 1); corr(s.c53, 4, 2); corr(s.c54, 4, 3); corr(s.c55, 4, 4);
-}
-
-// The parameters' part of the update: residuals nr = x - h and the negated gain.
-template <typename V, typename A>
-__device__ __forceinline__ void update_v2_params(Trk<V, A> &s, V hx, V hy, const V (&nK)[5][2]) {
-  const V nr0 = acc_nres(hx, s.x), nr1 = acc_nres(hy, s.y);
-  acc_kalman(s.x, hx, nK[0][0], nr0, nK[0][1], nr1);
-  acc_kalman(s.y, hy, nK[1][1], nr1, nK[1][0], nr0);
-  const V dphi = vfma(nK[3][1], nr1, vmul(nK[3][0], nr0));
-  const V dth = vfma(nK[4][1], nr1, vmul(nK[4][0], nr0));
-  phi_add(s.phi, dphi);
-  s.theta = vadd(s.theta, dth);
+// Joseph form of a track's first update (see above).
+template <typename A>
+__device__ __forceinline__ void update_v2_apply_joseph(Trk<float, A> &s, float i00, float i01, float i11, float hx,
+                                                       float hy, float v00, float v01, float v11) {
+  const float2 I0 = make_float2(i00, i01), I1 = make_float2(i01, i11);
+  const float2 A0 = make_float2(s.c00, s.c10), A1 = make_float2(s.c10, s.c11);
+  const float2 B3 = make_float2(s.c30, s.c31), B4 = make_float2(s.c40, s.c41), B5 = make_float2(s.c50, s.c51);
+  const float2 Kx = fma2(bc2(s.c10), I1, mul2(bc2(s.c00), I0));  // (K0, K1)
+  const float2 Ky = fma2(bc2(s.c11), I1, mul2(bc2(s.c10), I0));  // (K2, K3)
+  const float2 Ki = fma2(bc2(B3.y), I1, mul2(bc2(B3.x), I0));    // (K6, K7)
+  const float2 Kp = fma2(bc2(B4.y), I1, mul2(bc2(B4.x), I0));    // (K8, K9)
+  const float2 Kt = fma2(bc2(B5.y), I1, mul2(bc2(B5.x), I0));    // (K10, K11)
+  const float res0 = acc_res(hx, s.x), res1 = acc_res(hy, s.y);
+  acc_update(s.x, hx, res0, Kx.x * res0 + Kx.y * res1);
+  acc_update(s.y, hy, res1, Ky.x * res0 + Ky.y * res1);
+  const float dphi = Kp.x * res0 + Kp.y * res1;
+  const float dth = Kt.x * res0 + Kt.y * res1;
+  acc_add(s.phi, dphi);
+  s.theta = __fadd_rn(s.theta, dth);
   turn_direction(s, dphi, dth);
-  s.ipt = vfma(nK[2][1], nr1, vfma(nK[2][0], nr0, s.ipt));
-}
-
-// det(I - K H) = det(V)/det(R) at or below the limit: see kJosephShrink.
-// (n00, n01, n11): the negated inverse of R.
-__device__ __forceinline__ bool shrinks(float g) { return !(g > kJosephShrink); }
-__device__ __forceinline__ Bool2 shrinks(float2 g) { return {!(g.x > kJosephShrink), !(g.y > kJosephShrink)}; }
-__device__ __forceinline__ bool any(bool a) { return a; }
-__device__ __forceinline__ bool any(Bool2 a) { return a.x || a.y; }
-template <typename V>
-__device__ __forceinline__ V shrink(V n00, V n01, V n11, V v00, V v01, V v11) {
-  return vmul(vfma(v00, v11, vneg(vmul(v01, v01))), vfma(n00, n11, vneg(vmul(n01, n01))));
-}
-
-// The 2-D update from the negated inverse of R = H C H^T + V, two tracks:
-// nK(i,:) = (c_i0, c_i1) times it, c_ij' = c_ij + nK_i0 c_0j + nK_i1 c_1j.
-template <bool FIRST, typename A>
-__device__ __forceinline__ void update_v2_gain(Trk<float2, A> &s, float2 n00, float2 n01, float2 n11, float2 hx,
-                                               float2 hy, float2 v00, float2 v01, float2 v11) {
-  using V = float2;
-  const V c00 = s.c00, c10 = s.c10, c11 = s.c11, c30 = s.c30, c31 = s.c31, c40 = s.c40, c41 = s.c41;
-  const V c50 = s.c50, c51 = s.c51;
-  const V m0[5] = {c00, c10, c30, c40, c50}, m1[5] = {c10, c11, c31, c41, c51};
-  V nK[5][2];
-#pragma unroll
-  for (int i = 0; i < 5; ++i) nK[i][0] = vmul(n00, m0[i]);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) nK[i][1] = vmul(n01, m0[i]);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) nK[i][0] = vfma(n01, m1[i], nK[i][0]);
-#pragma unroll
-  for (int i = 0; i < 5; ++i) nK[i][1] = vfma(n11, m1[i], nK[i][1]);
-  update_v2_params(s, hx, hy, nK);
-  auto upd = [&](V c, int i, V c0, V c1) { return vfma(nK[i][1], c1, vfma(nK[i][0], c0, c)); };
-  {
-    V k = nK[0][0];
-    s.c00 = vfma(k, c00, c00);
-    k = nK[1][0];
-    s.c10 = vfma(k, c00, c10); s.c11 = vfma(k, c10, c11);
-    k = nK[2][0];
-    s.c30 = vfma(k, c00, c30); s.c31 = vfma(k, c10, c31); s.c33 = vfma(k, c30, s.c33);
-    k = nK[3][0];
-    s.c40 = vfma(k, c00, c40); s.c41 = vfma(k, c10, c41); s.c43 = vfma(k, c30, s.c43); s.c44 = vfma(k, c40, s.c44);
-    k = nK[4][0];
-    s.c50 = vfma(k, c00, c50); s.c51 = vfma(k, c10, c51); s.c53 = vfma(k, c30, s.c53); s.c54 = vfma(k, c40, s.c54);
-    s.c55 = vfma(k, c50, s.c55);
-    k = nK[0][1];
-    s.c00 = vfma(k, c10, s.c00);
-    k = nK[1][1];
-    s.c10 = vfma(k, c10, s.c10); s.c11 = vfma(k, c11, s.c11);
-    k = nK[2][1];
-    s.c30 = vfma(k, c10, s.c30); s.c31 = vfma(k, c11, s.c31); s.c33 = vfma(k, c31, s.c33);
-    k = nK[3][1];
-    s.c40 = vfma(k, c10, s.c40); s.c41 = vfma(k, c11, s.c41); s.c43 = vfma(k, c31, s.c43); s.c44 = vfma(k, c41, s.c44);
-    k = nK[4][1];
-    s.c50 = vfma(k, c10, s.c50); s.c51 = vfma(k, c11, s.c51); s.c53 = vfma(k, c31, s.c53); s.c54 = vfma(k, c41, s.c54);
-    s.c55 = vfma(k, c51, s.c55);
-  }
-  if constexpr (FIRST) {
-    const Bool2 j = shrinks(shrink(n00, n01, n11, v00, v01, v11));
-    if (any(j)) update_v2_joseph(s, j, upd(c10, 0, c10, c11), nK, v00, v01, v11);
-  }
-}
-
-// One track: the same operations with the column-0/1 pairs of rows y, ipt,
-// phi, theta in packed FP32 pairs.
-template <bool FIRST, typename A>
-__device__ __forceinline__ void update_v2_gain(Trk<float, A> &s, float n00, float n01, float n11, float hx, float hy,
-                                               float v00, float v01, float v11) {
-  const float2 N0 = make_float2(n00, n01), N1 = make_float2(n01, n11);
-  const float2 Kx = fma2(bc2(s.c10), N1, mul2(bc2(s.c00), N0));
-  const float2 Ky = fma2(bc2(s.c11), N1, mul2(bc2(s.c10), N0));
-  const float2 Ki = fma2(bc2(s.c31), N1, mul2(bc2(s.c30), N0));
-  const float2 Kp = fma2(bc2(s.c41), N1, mul2(bc2(s.c40), N0));
-  const float2 Kt = fma2(bc2(s.c51), N1, mul2(bc2(s.c50), N0));
-  const float nK[5][2] = {{Kx.x, Kx.y}, {Ky.x, Ky.y}, {Ki.x, Ki.y}, {Kp.x, Kp.y}, {Kt.x, Kt.y}};
-  update_v2_params(s, hx, hy, nK);
-  const float2 P0 = make_float2(s.c00, s.c10), Q = make_float2(s.c10, s.c11);
-  const float c30 = s.c30, c31 = s.c31, c40 = s.c40, c41 = s.c41, c50 = s.c50, c51 = s.c51;
-  const float p01 = FIRST ? vfma(Kx.y, Q.y, vfma(Kx.x, Q.x, Q.x)) : 0.f;
-  s.c00 = vfma(Kx.y, Q.x, vfma(Kx.x, P0.x, P0.x));
-  const float2 Ny = fma2(bc2(Ky.y), Q, fma2(bc2(Ky.x), P0, Q));
-  const float2 Ni = fma2(bc2(Ki.y), Q, fma2(bc2(Ki.x), P0, make_float2(c30, c31)));
-  const float2 Np = fma2(bc2(Kp.y), Q, fma2(bc2(Kp.x), P0, make_float2(c40, c41)));
-  const float2 Nt = fma2(bc2(Kt.y), Q, fma2(bc2(Kt.x), P0, make_float2(c50, c51)));
+  s.ipt = s.ipt + Ki.x * res0 + Ki.y * res1;
+  // P = C - K H C on the measured columns of every live row
+  const float2 Px = fma2(bc2(-Kx.y), A1, fma2(bc2(-Kx.x), A0, A0));
+  const float2 Py = fma2(bc2(-Ky.y), A1, fma2(bc2(-Ky.x), A0, A1));
+  const float2 Pi = fma2(bc2(-Ki.y), A1, fma2(bc2(-Ki.x), A0, B3));
+  const float2 Pp = fma2(bc2(-Kp.y), A1, fma2(bc2(-Kp.x), A0, B4));
+  const float2 Pt = fma2(bc2(-Kt.y), A1, fma2(bc2(-Kt.x), A0, B5));
+  // E_i = P_i - K_i V (K V from error-free products), then
+  // C''(i, m) = P(i, m) - E_i . K_m for the measured columns and
+  // C''(a, b) = C(a, b) - K_a . B_b - E_a . K_b on the unmeasured block.
+  const float2 V0 = make_float2(v00, v01), V1 = make_float2(v01, v11);
+  const float2 Kc0 = make_float2(Kx.x, Ky.x), Kc1 = make_float2(Kx.y, Ky.y);
+  auto resid = [&](const float2 P, const float2 K) {
+    const float2 p = mul2(bc2(-K.x), V0);
+    const float2 e = fma2(bc2(-K.x), V0, make_float2(-p.x, -p.y));  // exact: -K0 V0 - p
+    return __fadd2_rn(__fadd2_rn(fma2(bc2(-K.y), V1, p), e), P);
+  };
+  const float2 Ex = resid(Px, Kx), Ey = resid(Py, Ky), Ei = resid(Pi, Ki), Ep = resid(Pp, Kp), Et = resid(Pt, Kt);
+  const float2 Nx = fma2(bc2(-Ex.y), Kc1, fma2(bc2(-Ex.x), Kc0, Px));
+  const float2 Ny = fma2(bc2(-Ey.y), Kc1, fma2(bc2(-Ey.x), Kc0, Py));
+  const float2 Ni = fma2(bc2(-Ei.y), Kc1, fma2(bc2(-Ei.x), Kc0, Pi));
+  const float2 Np = fma2(bc2(-Ep.y), Kc1, fma2(bc2(-Ep.x), Kc0, Pp));
+  const float2 Nt = fma2(bc2(-Et.y), Kc1, fma2(bc2(-Et.x), Kc0, Pt));
+  s.c33 = fmaf(-Ei.y, Ki.y, fmaf(-Ei.x, Ki.x, fmaf(-Ki.y, B3.y, fmaf(-Ki.x, B3.x, s.c33))));
+  s.c43 = fmaf(-Ep.y, Ki.y, fmaf(-Ep.x, Ki.x, fmaf(-Kp.y, B3.y, fmaf(-Kp.x, B3.x, s.c43))));
+  s.c44 = fmaf(-Ep.y, Kp.y, fmaf(-Ep.x, Kp.x, fmaf(-Kp.y, B4.y, fmaf(-Kp.x, B4.x, s.c44))));
+  s.c53 = fmaf(-Et.y, Ki.y, fmaf(-Et.x, Ki.x, fmaf(-Kt.y, B3.y, fmaf(-Kt.x, B3.x, s.c53))));
+  s.c54 = fmaf(-Et.y, Kp.y, fmaf(-Et.x, Kp.x, fmaf(-Kt.y, B4.y, fmaf(-Kt.x, B4.x, s.c54))));
+  s.c55 = fmaf(-Et.y, Kt.y, fmaf(-Et.x, Kt.x, fmaf(-Kt.y, B5.y, fmaf(-Kt.x, B5.x, s.c55))));
+  s.c00 = Nx.x;
   s.c10 = Ny.x; s.c11 = Ny.y;
   s.c30 = Ni.x; s.c31 = Ni.y;
   s.c40 = Np.x; s.c41 = Np.y;
   s.c50 = Nt.x; s.c51 = Nt.y;
-  s.c33 = vfma(Ki.y, c31, vfma(Ki.x, c30, s.c33));
-  s.c43 = vfma(Kp.y, c31, vfma(Kp.x, c30, s.c43));
-  s.c44 = vfma(Kp.y, c41, vfma(Kp.x, c40, s.c44));
-  s.c53 = vfma(Kt.y, c31, vfma(Kt.x, c30, s.c53));
-  s.c54 = vfma(Kt.y, c41, vfma(Kt.x, c40, s.c54));
-  s.c55 = vfma(Kt.y, c51, vfma(Kt.x, c50, s.c55));
+}
+
+// Every later update: the reference's C - K H C with the column-0/1 pairs of
+// rows y, ipt, phi, theta updated together:
+//   (c_i0, c_i1)' = (c_i0, c_i1) - K_i0 (c00, c10) - K_i1 (c10, c11).
+template <bool FIRST, typename A>
+__device__ __forceinline__ void update_v2_apply_packed(Trk<float, A> &s, float r00, float r01, float r11, float hx,
+                                                       float hy, float v00, float v01, float v11) {
   if constexpr (FIRST) {
-    const bool j = shrinks(shrink(n00, n01, n11, v00, v01, v11));
-    if (j) update_v2_joseph(s, true, p01, nK, v00, v01, v11);
+    // shrink test: det(I - K H) = det(V) / det(R), and r00 r11 - r01^2 = 1/det(R)
+    const float g = fmaf(v00, v11, -(v01 * v01)) * fmaf(r00, r11, -(r01 * r01));
+    if (!(g > kJosephShrink)) {
+      update_v2_apply_joseph(s, r00, r01, r11, hx, hy, v00, v01, v11);
+      return;
+    }
   }
+  (void)v00;
+  (void)v01;
+  (void)v11;
+  const float2 R0 = make_float2(r00, r01), R1 = make_float2(r01, r11);
+  const float2 Kx = fma2(bc2(s.c10), R1, mul2(bc2(s.c00), R0));  // (K0, K1)
+  const float2 Ky = fma2(bc2(s.c11), R1, mul2(bc2(s.c10), R0));  // (K2, K3)
+  const float2 Ki = fma2(bc2(s.c31), R1, mul2(bc2(s.c30), R0));  // (K6, K7)
+  const float2 Kp = fma2(bc2(s.c41), R1, mul2(bc2(s.c40), R0));  // (K8, K9)
+  const float2 Kt = fma2(bc2(s.c51), R1, mul2(bc2(s.c50), R0));  // (K10, K11)
+  const float res0 = acc_res(hx, s.x), res1 = acc_res(hy, s.y);
+  acc_update(s.x, hx, res0, Kx.x * res0 + Kx.y * res1);
+  acc_update(s.y, hy, res1, Ky.x * res0 + Ky.y * res1);
+  const float dphi = Kp.x * res0 + Kp.y * res1;
+  const float dth = Kt.x * res0 + Kt.y * res1;
+  acc_add(s.phi, dphi);
+  s.theta = __fadd_rn(s.theta, dth);
+  turn_direction(s, dphi, dth);
+  s.ipt = s.ipt + Ki.x * res0 + Ki.y * res1;
+  const float2 P0 = make_float2(s.c00, s.c10), Q = make_float2(s.c10, s.c11);
+  const float c30 = s.c30, c31 = s.c31, c40 = s.c40, c41 = s.c41, c50 = s.c50, c51 = s.c51;
+  s.c00 = fmaf(-Kx.y, s.c10, fmaf(-Kx.x, s.c00, s.c00));
+  const float2 Ny = fma2(bc2(-Ky.y), Q, fma2(bc2(-Ky.x), P0, Q));
+  const float2 Ni = fma2(bc2(-Ki.y), Q, fma2(bc2(-Ki.x), P0, make_float2(c30, c31)));
+  const float2 Np = fma2(bc2(-Kp.y), Q, fma2(bc2(-Kp.x), P0, make_float2(c40, c41)));
+  const float2 Nt = fma2(bc2(-Kt.y), Q, fma2(bc2(-Kt.x), P0, make_float2(c50, c51)));
+  s.c10 = Ny.x; s.c11 = Ny.y;
+  s.c30 = Ni.x; s.c31 = Ni.y;
+  s.c40 = Np.x; s.c41 = Np.y;
+  s.c50 = Nt.x; s.c51 = Nt.y;
+  s.c33 = fmaf(-Ki.y, c31, fmaf(-Ki.x, c30, s.c33));
+  s.c43 = fmaf(-Kp.y, c31, fmaf(-Kp.x, c30, s.c43));
+  s.c44 = fmaf(-Kp.y, c41, fmaf(-Kp.x, c40, s.c44));
+  s.c53 = fmaf(-Kt.y, c31, fmaf(-Kt.x, c30, s.c53));
+  s.c54 = fmaf(-Kt.y, c41, fmaf(-Kt.x, c40, s.c54));
+  s.c55 = fmaf(-Kt.y, c51, fmaf(-Kt.x, c50, s.c55));
 }
 
-// The precise 2-D update: R = C(xy) + V(xy), Kahan's compensated FP32
-// determinant (error <= 2 ulp of the exact determinant of the float entries,
-// the same bound as the FP64 product rounded to float) and a Newton-refined
-// reciprocal -- no FP64.  live: a track that has no step left keeps its state
-// (zero gain).  Returns true when a live track's det is <= 0 or NaN.
-__device__ __forceinline__ bool not_positive(float d, bool live) { return live && !(d > 0.0f); }
-__device__ __forceinline__ bool not_positive(float2 d, Bool2 live) {
-  return (live.x && !(d.x > 0.0f)) || (live.y && !(d.y > 0.0f));
-}
-template <bool FIRST, typename V, typename A, typename L>
-__device__ __forceinline__ bool update_v2_precise(Trk<V, A> &s, V hx, V hy, V v00, V v01, V v11, L live) {
-  const V r00 = vadd(s.c00, v00), r01 = vadd(s.c10, v01), r11 = vadd(s.c11, v11);
-  // det = r00 r11 - r01^2: w = -r01^2 rounded, e = its error, exactly
-  const V nr01 = vneg(r01);
-  const V w = vmul(nr01, r01);
-  const V e = vfma(r01, r01, w);
-  const V det = vsub(vfma(r00, r11, w), e);
-  const V nsc = vsel(live, nrcp_nr(det), vset<V>(0.f));
-  update_v2_gain<FIRST>(s, vmul(nsc, r11), vmul(nsc, nr01), vmul(nsc, r00), hx, hy, v00, v01, v11);
-  return not_positive(det, live);
-}
-
-// The generic form (FP64 kernel, reference rounding): the reference's C - K (H C).
-template <typename T, typename A>
-__device__ __forceinline__ void update_v2_apply(Trk<T, A> &s, T r00, T r01, T r11, T hx, T hy) {
+// The generic form (FP64 kernel, reference rounding, unpacked FP32): the
+// reference's C - K (H C).  v (the hit covariance) is used by the packed FP32
+// form only.
+template <typename T, typename A, int FORM, bool FIRST = false>
+__device__ __forceinline__ void update_v2_apply(Trk<T, A> &s, T r00, T r01, T r11, T hx, T hy, const T (&v)[3]) {
+  if constexpr (P2Z_PACKED_F32X2 && FORM == FORM_PRECISE && std::is_same<T, float>::value) {
+    update_v2_apply_packed<FIRST>(s, r00, r01, r11, hx, hy, v[0], v[1], v[2]);
+    return;
+  }
+  (void)v;
   const T K0 = s.c00 * r00 + s.c10 * r01, K1 = s.c00 * r01 + s.c10 * r11;
   const T K2 = s.c10 * r00 + s.c11 * r01, K3 = s.c10 * r01 + s.c11 * r11;
   const T K6 = s.c30 * r00 + s.c31 * r01, K7 = s.c30 * r01 + s.c31 * r11;
   const T K8 = s.c40 * r00 + s.c41 * r01, K9 = s.c40 * r01 + s.c41 * r11;
   const T K10 = s.c50 * r00 + s.c51 * r01, K11 = s.c50 * r01 + s.c51 * r11;
   const T res0 = acc_res(hx, s.x), res1 = acc_res(hy, s.y);
-  if constexpr (std::is_same<T, float>::value) {
+  if constexpr (FORM == FORM_REFERENCE) {
     // reference order: p + K0*r0 + K1*r1, left to right
     acc_set(s.x, tof(s.x) + K0 * res0 + K1 * res1);
     acc_set(s.y, tof(s.y) + K2 * res0 + K3 * res1);
     acc_set(s.phi, tof(s.phi) + K8 * res0 + K9 * res1);
     s.theta = s.theta + K10 * res0 + K11 * res1;
+  } else if constexpr (std::is_same<T, float>::value) {
+    acc_update(s.x, hx, res0, K0 * res0 + K1 * res1);
+    acc_update(s.y, hy, res1, K2 * res0 + K3 * res1);
+    const float dphi = K8 * res0 + K9 * res1;
+    const float dth = K10 * res0 + K11 * res1;
+    acc_add(s.phi, dphi);
+    s.theta = __fadd_rn(s.theta, dth);
+    turn_direction(s, dphi, dth);
   } else {
     acc_add(s.x, K0 * res0 + K1 * res1);
     acc_add(s.y, K2 * res0 + K3 * res1);
@@ -1191,42 +885,78 @@ __device__ __forceinline__ void update_v2_apply(Trk<T, A> &s, T r00, T r01, T r1
     s.theta = s.theta + K10 * res0 + K11 * res1;
   }
   s.ipt = s.ipt + K6 * res0 + K7 * res1;
-  const T e0 = K0 * s.c00 + K1 * s.c10;
-  const T e1 = K2 * s.c00 + K3 * s.c10;
-  const T e2 = K2 * s.c10 + K3 * s.c11;
-  const T e6 = K6 * s.c00 + K7 * s.c10;
-  const T e7 = K6 * s.c10 + K7 * s.c11;
-  const T e9 = K6 * s.c30 + K7 * s.c31;
-  const T e10 = K8 * s.c00 + K9 * s.c10;
-  const T e11 = K8 * s.c10 + K9 * s.c11;
-  const T e13 = K8 * s.c30 + K9 * s.c31;
-  const T e14 = K8 * s.c40 + K9 * s.c41;
-  const T e15 = K10 * s.c00 + K11 * s.c10;
-  const T e16 = K10 * s.c10 + K11 * s.c11;
-  const T e18 = K10 * s.c30 + K11 * s.c31;
-  const T e19 = K10 * s.c40 + K11 * s.c41;
-  const T e20 = K10 * s.c50 + K11 * s.c51;
-  s.c00 = s.c00 - e0;  s.c10 = s.c10 - e1;  s.c11 = s.c11 - e2;
-  s.c30 = s.c30 - e6;  s.c31 = s.c31 - e7;  s.c33 = s.c33 - e9;
-  s.c40 = s.c40 - e10; s.c41 = s.c41 - e11; s.c43 = s.c43 - e13; s.c44 = s.c44 - e14;
-  s.c50 = s.c50 - e15; s.c51 = s.c51 - e16; s.c53 = s.c53 - e18; s.c54 = s.c54 - e19; s.c55 = s.c55 - e20;
+  if constexpr (FORM == FORM_PRECISE && std::is_same<T, float>::value) {
+    // C - K (H C), each element as two fused multiply-adds: C - K_i0 C_0j - K_i1 C_1j
+    const T c00 = s.c00, c10 = s.c10, c11 = s.c11, c30 = s.c30, c31 = s.c31, c40 = s.c40, c41 = s.c41;
+    const T c50 = s.c50, c51 = s.c51;
+    s.c00 = fmaf(-K1, c10, fmaf(-K0, c00, c00));
+    s.c10 = fmaf(-K3, c10, fmaf(-K2, c00, c10));
+    s.c11 = fmaf(-K3, c11, fmaf(-K2, c10, c11));
+    s.c30 = fmaf(-K7, c10, fmaf(-K6, c00, c30));
+    s.c31 = fmaf(-K7, c11, fmaf(-K6, c10, c31));
+    s.c33 = fmaf(-K7, c31, fmaf(-K6, c30, s.c33));
+    s.c40 = fmaf(-K9, c10, fmaf(-K8, c00, c40));
+    s.c41 = fmaf(-K9, c11, fmaf(-K8, c10, c41));
+    s.c43 = fmaf(-K9, c31, fmaf(-K8, c30, s.c43));
+    s.c44 = fmaf(-K9, c41, fmaf(-K8, c40, s.c44));
+    s.c50 = fmaf(-K11, c10, fmaf(-K10, c00, c50));
+    s.c51 = fmaf(-K11, c11, fmaf(-K10, c10, c51));
+    s.c53 = fmaf(-K11, c31, fmaf(-K10, c30, s.c53));
+    s.c54 = fmaf(-K11, c41, fmaf(-K10, c40, s.c54));
+    s.c55 = fmaf(-K11, c51, fmaf(-K10, c50, s.c55));
+  } else {
+    const T e0 = K0 * s.c00 + K1 * s.c10;
+    const T e1 = K2 * s.c00 + K3 * s.c10;
+    const T e2 = K2 * s.c10 + K3 * s.c11;
+    const T e6 = K6 * s.c00 + K7 * s.c10;
+    const T e7 = K6 * s.c10 + K7 * s.c11;
+    const T e9 = K6 * s.c30 + K7 * s.c31;
+    const T e10 = K8 * s.c00 + K9 * s.c10;
+    const T e11 = K8 * s.c10 + K9 * s.c11;
+    const T e13 = K8 * s.c30 + K9 * s.c31;
+    const T e14 = K8 * s.c40 + K9 * s.c41;
+    const T e15 = K10 * s.c00 + K11 * s.c10;
+    const T e16 = K10 * s.c10 + K11 * s.c11;
+    const T e18 = K10 * s.c30 + K11 * s.c31;
+    const T e19 = K10 * s.c40 + K11 * s.c41;
+    const T e20 = K10 * s.c50 + K11 * s.c51;
+    s.c00 = s.c00 - e0;  s.c10 = s.c10 - e1;  s.c11 = s.c11 - e2;
+    s.c30 = s.c30 - e6;  s.c31 = s.c31 - e7;  s.c33 = s.c33 - e9;
+    s.c40 = s.c40 - e10; s.c41 = s.c41 - e11; s.c43 = s.c43 - e13; s.c44 = s.c44 - e14;
+    s.c50 = s.c50 - e15; s.c51 = s.c51 - e16; s.c53 = s.c53 - e18; s.c54 = s.c54 - e19; s.c55 = s.c55 - e20;
+  }
 }
 
-// KalmanUpdate_v2 (reference :503-620) in the reference's own rounding: R =
-// C(xy) + V(xy), the determinant in FP64 from the float entries and 1.f/det as
-// a double division rounded to float.  Returns true when det <= 0 (or NaN).
-__device__ __forceinline__ bool update_v2_ref(Trk<float, float> &s, const float (&hp)[3], const float (&hc)[3]) {
+// KalmanUpdate_v2 (reference :503-620): R = C(xy) + V(xy), its inverse by
+// Cramer's rule, gain, parameter and covariance update.
+// FORM_REFERENCE: the determinant in FP64 from the float entries and 1.f/det as
+// a double division rounded to float, as the reference.
+// FORM_PRECISE: Kahan's compensated FP32 determinant (error <= 2 ulp of the
+// exact determinant of the float entries, the same bound as the FP64 product
+// rounded to float) and a correctly rounded float reciprocal -- no FP64.
+// Returns true when det <= 0 (or NaN).
+template <typename A, int FORM, bool FIRST = false>
+__device__ __forceinline__ bool update_v2(Trk<float, A> &s, const float (&hp)[3], const float (&hc)[3]) {
   float r00 = s.c00 + hc[0];
   float r01 = s.c10 + hc[1];
   float r11 = s.c11 + hc[2];
-  const double det = (double)r00 * r11 - (double)r01 * r01;
-  const float sc = 1.f / det;
+  float sc;
+  bool bad;
+  if constexpr (FORM == FORM_REFERENCE) {
+    const double det = (double)r00 * r11 - (double)r01 * r01;
+    sc = 1.f / det;
+    bad = !(det > 0.0);
+  } else {
+    const float det = det2_comp(r00, r01, r01, r11);
+    sc = rcp_nr(det);
+    bad = !(det > 0.0f);
+  }
   const float tmp = sc * r11;
   r01 *= -sc;
   r11 = sc * r00;
   r00 = tmp;
-  update_v2_apply<float, float>(s, r00, r01, r11, hp[0], hp[1]);
-  return !(det > 0.0);
+  update_v2_apply<float, A, FORM, FIRST>(s, r00, r01, r11, hp[0], hp[1], hc);
+  return bad;
 }
 
 // FP64 2-D update for the all-FP64 kernel.
@@ -1234,7 +964,7 @@ __device__ __forceinline__ bool update_v2_f64(Trk<double, double> &s, const doub
   const double r00 = s.c00 + hc[0], r01 = s.c10 + hc[1], r11 = s.c11 + hc[2];
   const double det = r00 * r11 - r01 * r01;
   const double id = 1.0 / det;
-  update_v2_apply<double, double>(s, r11 * id, -r01 * id, r00 * id, hp[0], hp[1]);
+  update_v2_apply<double, double, FORM_PRECISE>(s, r11 * id, -r01 * id, r00 * id, hp[0], hp[1], hc);
   return !(det > 0.0);
 }
 

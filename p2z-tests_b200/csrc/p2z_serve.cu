@@ -199,7 +199,6 @@ void launch_group(p2z_server *s) {
   LaunchSpec spec;
   std::memset(&spec, 0, sizeof spec);
   spec.tpt = 1;
-  spec.duo = -1;
   spec.early = false;
   spec.args.trk = s->d_trk;
   spec.args.hits = s->d_hit;

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) k_step(float *trk, const float *hits, int
     s.x = p[0]; s.y = p[1]; s.z = p[2]; s.ipt = p[3]; s.phi = p[4]; s.theta = p[5];
     const Helix<float> hx = propagate_params_ref(s, hpos[2], k);
     const Jac<float> J = jacobian_ref(hx, k, s.ipt);
-    propagate_cov_general(s, C, J);
+    propagate_cov_general(s, C, hx, J);
     p[0] = s.x; p[1] = s.y; p[2] = s.z; p[3] = s.ipt; p[4] = s.phi; p[5] = s.theta;
     C[0] = s.c00; C[1] = s.c10; C[2] = s.c11; C[3] = 0.f; C[4] = 0.f; C[5] = 0.f;
     C[6] = s.c30; C[7] = s.c31; C[8] = 0.f; C[9] = s.c33;
