@@ -305,10 +305,8 @@ def tune_summary(best, rows, wall_s):
 def small_run_latency(p2z, ctx, t, h, o):
     """Host wall time of one synchronous p2z_run call on a lone event of 1024
     or 9600 tracks from page-locked buffers (the first batches of the bench
-    sample): the default call -- a pipeline of 4 or more chunk passes (9600
-    tracks: 4 chunks) replayed as a recorded graph, a shorter one (1024
-    tracks: 1 chunk) enqueued directly -- against the same pipeline always
-    enqueued copy by copy (P2Z_FLAG_NO_GRAPH); mean of 200 calls after 5
+    sample), one pass across the link: the default call and the same with
+    P2Z_FLAG_NO_GRAPH, which changes nothing here; mean of 200 calls after 5
     warm-up calls."""
     out = {}
     for n in (1024, 9600):
@@ -327,8 +325,7 @@ def small_run_latency(p2z, ctx, t, h, o):
                 raise p2z.P2zError(rc, p2z.lib.p2z_last_error(ctx.h).decode())
             row[mode + "_us"] = us
         out[str(n)] = row
-    return {"note": "p2z_run from page-locked buffers, one event, host wall time per synchronous call; default: "
-                    "recorded graph from 4 chunk passes (9600 tracks), direct below (1024 tracks)",
+    return {"note": "p2z_run from page-locked buffers, one event, host wall time per synchronous call",
             "tracks": out}
 
 
