@@ -109,10 +109,16 @@ constexpr int kSortWindow = 128;
 // One B200, 2-D update, us per pass, stored order / sorted: 51,000 tracks 18.6 /
 // 20.8, 102,000 30.7 / 30.8, 152,000 41.0 / 39.2, 406,000 88.1 / 81.6.
 constexpr int64_t kSortMinSlotsPerSm = 768;
+// A warp's counts of one group of 32 slots, a byte a key (0..32), cleared by words.
+union KeyCounts {
+  uint32_t word[9];
+  uint8_t of[36];
+};
+static_assert(alignof(KeyCounts) == alignof(uint32_t) && sizeof(KeyCounts) == 36, "cleared by 4-byte stores");
 __device__ __forceinline__ int sorted_offset(const uint32_t *__restrict__ mask, int64_t base, int n, int rank,
                                              uint32_t all) {
   constexpr int G = kSortWindow / 32;
-  __shared__ uint8_t s_count[8][G][36];  // per warp: slots of each key in each group of 32
+  __shared__ KeyCounts s_count[8][G];  // per warp and group
   __shared__ uint8_t s_order[8][32];
   const int lane = threadIdx.x & 31;
   auto &count = s_count[threadIdx.x >> 5];
@@ -122,15 +128,13 @@ __device__ __forceinline__ int sorted_offset(const uint32_t *__restrict__ mask, 
 #pragma unroll
   for (int g = 0; g < G; ++g) key[g] = 32 * g + lane < n ? 32 - __popc(__ldg(mask + base + 32 * g + lane) & all) : 32;
 #pragma unroll
-  for (int g = 0; g < G; ++g) {
-    reinterpret_cast<uint32_t *>(count[g])[min(lane, 8)] = 0u;
-  }
+  for (int g = 0; g < G; ++g) count[g].word[min(lane, 8)] = 0u;
   __syncwarp();
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     const unsigned same = __match_any_sync(0xffffffffu, key[g]);
     in_group[g] = __popc(same & ((1u << lane) - 1u));
-    if (in_group[g] == 0) count[g][key[g]] = (uint8_t)__popc(same);
+    if (in_group[g] == 0) count[g].of[key[g]] = (uint8_t)__popc(same);
   }
   __syncwarp();
   // lane k: the slots with keys below k, then those with key k in earlier groups
@@ -138,7 +142,7 @@ __device__ __forceinline__ int sorted_offset(const uint32_t *__restrict__ mask, 
 #pragma unroll
   for (int g = 0; g < G; ++g) {
     of_key[g] = total;
-    total += count[g][lane];
+    total += count[g].of[lane];
   }
   int below = total;
 #pragma unroll
@@ -154,7 +158,7 @@ __device__ __forceinline__ int sorted_offset(const uint32_t *__restrict__ mask, 
     const int from = __shfl_sync(0xffffffffu, below + of_key[g], key[g] & 31);
     const int pos = (key[g] < 32 ? from : last + before32) + in_group[g] - (rank & ~31);
     if (pos >= 0 && pos < 32) order[pos] = (uint8_t)(32 * g + lane);
-    before32 += count[g][32];
+    before32 += count[g].of[32];
   }
   __syncwarp();
   return order[rank & 31];
