@@ -286,7 +286,8 @@ size_t p2z_sizeof_mphit(int bsize);   /* 9*bsize*4 */
  * Host buffers that are page-locked (cudaHostAlloc / p2z_host_alloc) are
  * copied asynchronously; pageable ones go through a staging path.  The work is
  * split into up to 16 chunks: the copies in follow one another on one stream,
- * each chunk's pass and its copy back on another.  With page-locked buffers, no
+ * each chunk's pass and its copy back on another.  With buffers that are
+ * page-locked throughout, start on 4-byte boundaries and do not overlap trk_out, no
  * hit mask, at most 256 MB of input, bsize 32 or 64 or the SoA layout, and none of
  * the PER_EVENT schedule, P2Z_FLAG_CHECK_INPUTS and P2Z_FLAG_FULL_HITS, there
  * are no copies: one pass reads and writes the host arrays over the link.

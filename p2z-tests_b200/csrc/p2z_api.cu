@@ -1,6 +1,7 @@
 // p2z_api.cu -- the extern "C" boundary (include/p2z.h): contexts, the hot-path
 // run entry points, launch scheduling (flat / per-event / persistent replayed
 // as a CUDA graph) and host<->device copy pipelining.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -13,6 +14,7 @@
 #include <vector>
 
 #include "p2z.h"
+#include "p2z_direct.h"
 #include "p2z_kernels.cuh"
 
 // p2z_run: the host->device copies and the passes are pipelined over chunks, each
@@ -287,15 +289,34 @@ p2z_status event_streams(p2z_context *ctx) {
   return P2Z_OK;
 }
 
-// The device's address of page-locked host memory (cudaHostAlloc, or
-// cudaHostRegister where the device can reach it), else null.
-float *mapped_host(const void *p) {
+// The page-locked range (cudaHostAlloc, or cudaHostRegister where the device can
+// reach it) that holds a host address; false where there is none or its extent is not known.
+bool page_locked_range(uintptr_t p, HostRange *r) {
+  using GetAttribute = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const GetAttribute get = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return (GetAttribute)f;
+  }();
   cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+  if (!get || cudaPointerGetAttributes(&a, (const void *)p) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
+    return false;
   }
-  return a.type == cudaMemoryTypeHost ? (float *)a.devicePointer : nullptr;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer ||
+      get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS || (uintptr_t)start > p ||
+      (uintptr_t)start + size <= p)
+    return false;
+  *r = {(uintptr_t)start, (uintptr_t)start + size, (uintptr_t)a.devicePointer - (p - (uintptr_t)start)};
+  return true;
 }
 
 // Enqueue the hot-path launches of one pass over slots [s0, s1) on st.
@@ -834,14 +855,14 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
                    !(pl.flags & P2Z_FLAG_FULL_HITS);
   const size_t read_bytes = trk_bytes + hit_bytes / 9 * (six ? 6 : 9);
   // Page-locked arrays, every layer present: one pass reads and writes them over the
-  // link itself (see kRunDirectBytes).
-  const float *h_trk = nullptr, *h_hits = nullptr;
-  float *h_out = nullptr;
+  // link itself (see kRunDirectBytes and p2z_direct.h).
+  uintptr_t h_trk = 0, h_hits = 0, h_out = 0;
   if (pl.nslots > 0 && !user_mask && !check && !per_event && !(pl.flags & P2Z_FLAG_FULL_HITS) &&
-      (pl.soa || pl.B >= 32) && read_bytes <= kRunDirectBytes) {
-    h_trk = mapped_host(trk_in);
-    h_hits = mapped_host(hits);
-    h_out = mapped_host(trk_out);
+      (pl.soa || pl.B >= 32) && read_bytes <= kRunDirectBytes && !overlap(trk_out, trk_bytes, trk_in, trk_bytes) &&
+      !overlap(trk_out, trk_bytes, hits, hit_bytes)) {
+    h_trk = mapped_array(trk_in, trk_bytes, page_locked_range);
+    h_hits = mapped_array(hits, hit_bytes, page_locked_range);
+    h_out = mapped_array(trk_out, trk_bytes, page_locked_range);
   }
   const bool direct = h_trk && h_hits && h_out;
   if (!direct) {
@@ -852,9 +873,9 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
   pl.host = direct;
   RunArgs base;
   std::memset(&base, 0, sizeof base);
-  base.trk = direct ? h_trk : (const float *)ctx->trk.p;
-  base.hits = direct ? h_hits : (const float *)ctx->hits.p;
-  base.out = direct ? h_out : (float *)ctx->out.p;
+  base.trk = direct ? (const float *)h_trk : (const float *)ctx->trk.p;
+  base.hits = direct ? (const float *)h_hits : (const float *)ctx->hits.p;
+  base.out = direct ? (float *)h_out : (float *)ctx->out.p;
   base.mask = d_mask;
   base.nlayer = pl.nlayer;
   base.kfact = pl.kfact;
