@@ -208,7 +208,8 @@ typedef struct p2z_config {
                             this context for the same key, else the rule under p2z_schedule */
   int32_t block_threads; /* threads per CTA, a multiple of 32 in 32..256; 0 -> the value
                             p2z_autotune measured best on this context for the same update,
-                            flags, bsize, layout and masking, else 32 (FLAT, PER_EVENT),
+                            flags, bsize, layout and masking (no mask, uneven events without
+                            one, a caller's mask), else 32 (FLAT, PER_EVENT),
                             128 (other schedules, sorted windows) */
   uint32_t flags;        /* P2Z_FLAG_*; any other bit is P2Z_BAD_ARG */
   int32_t layout;        /* p2z_layout of the track, hit and output arrays */

@@ -16,6 +16,7 @@
 #include "p2z.h"
 #include "p2z_direct.h"
 #include "p2z_kernels.cuh"
+#include "p2z_shape.h"
 
 // p2z_run: the host->device copies and the passes are pipelined over chunks, each
 // a third of what is left but no less than 64 batches and 1/64 of the run: a copy
@@ -65,14 +66,6 @@ struct GraphKey {
   int bsize, upd, sc, block, grid, kind, tpt;
   bool masked, soa;
   bool operator==(const GraphKey &o) const { return std::memcmp(this, &o, sizeof(GraphKey)) == 0; }
-};
-
-// Launch shape p2z_autotune measured fastest for one kind of run.
-struct Tuned {
-  int upd, sc, B;
-  bool soa, masked;
-  int block, schedule, tpt;
-  bool sort;  // P2Z_FLAG_SORT_WINDOWS
 };
 
 }  // namespace
@@ -452,31 +445,21 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   return P2Z_OK;
 }
 
-// Applies the autotuner's measurement for this kind of run to the fields the
-// caller left open (block_threads = 0, schedule = AUTO -- with the window
-// sorting measured with that schedule --, threads_per_track = 0), then
-// resolves AUTO.  A tuned shape whose schedule the caller overrides
-// with STAGED keeps one thread per track.
-int resolve_schedule(p2z_context *ctx, Plan &pl, const p2z_config *cfg, bool masked) {
-  masked = masked || pl.uneven;
-  if (ctx) {
-    for (const Tuned &t : ctx->tuned) {
-      if (t.upd == pl.upd && t.sc == pl.sc && t.B == pl.B && t.soa == pl.soa && t.masked == masked) {
-        if (cfg->block_threads == 0) pl.block = t.block;
-        if (pl.schedule == P2Z_SCHED_AUTO) {
-          pl.schedule = t.schedule;
-          if (t.sort) pl.flags |= P2Z_FLAG_SORT_WINDOWS;
-        }
-        if (cfg->threads_per_track == 0 && pl.schedule != P2Z_SCHED_STAGED) pl.tpt = t.tpt;
-        break;
-      }
-    }
-  }
-  if (pl.schedule != P2Z_SCHED_AUTO) return pl.schedule;
-  // one flat launch; of large runs with a caller's mask the windows are sorted (see sorted_offset)
-  if (masked && pl.padding_mask == nullptr && ctx && pl.nslots >= ctx->num_sms * kSortMinSlotsPerSm)
-    pl.flags |= P2Z_FLAG_SORT_WINDOWS;
-  return P2Z_SCHED_FLAT;
+RunKind run_kind(const Plan &pl, bool caller_mask) {
+  return {pl.upd, pl.sc, pl.B, pl.soa, caller_mask ? MASK_CALLER : (pl.uneven ? MASK_PADDING : MASK_NONE)};
+}
+
+// Settles what the config leaves open (choose_shape); returns the schedule.
+int resolve_schedule(const p2z_context *ctx, Plan &pl, const p2z_config *cfg, bool caller_mask) {
+  const Shape s = choose_shape(ctx->tuned, run_kind(pl, caller_mask),
+                               {cfg->block_threads, cfg->schedule, cfg->threads_per_track,
+                                (pl.flags & P2Z_FLAG_SORT_WINDOWS) != 0},
+                               pl.nslots, ctx->num_sms);
+  pl.block = s.block;
+  pl.schedule = s.schedule;
+  pl.tpt = s.tpt;
+  if (s.sort) pl.flags |= P2Z_FLAG_SORT_WINDOWS;
+  return pl.schedule;
 }
 
 // Hit words an update kind reads per present layer: the 2-D updates the first
@@ -596,20 +579,11 @@ p2z_status context_fail(p2z_context *ctx, p2z_status st, const char *msg) { retu
 void *context_scratch(p2z_context *ctx, size_t bytes) {
   return ensure(ctx, ctx->aux, bytes) == P2Z_OK ? ctx->aux.p : nullptr;
 }
-p2z_status record_tuned(p2z_context *ctx, const p2z_config *cfg, bool masked, int block, int schedule, int tpt,
-                        bool sort) {
+p2z_status record_tuned(p2z_context *ctx, const p2z_config *cfg, bool caller_mask, const Shape &shape) {
   Plan pl;
   p2z_status r = make_plan(ctx, cfg, pl);
-  if (r != P2Z_OK) return r;
-  Tuned t{pl.upd, pl.sc, pl.B, pl.soa, masked || pl.uneven, block, schedule, tpt, sort};
-  for (Tuned &o : ctx->tuned) {
-    if (o.upd == t.upd && o.sc == t.sc && o.B == t.B && o.soa == t.soa && o.masked == t.masked) {
-      o = t;
-      return P2Z_OK;
-    }
-  }
-  ctx->tuned.push_back(t);
-  return P2Z_OK;
+  if (r == P2Z_OK) record_shape(ctx->tuned, run_kind(pl, caller_mask), shape);
+  return r;
 }
 }  // namespace p2z
 
@@ -769,7 +743,7 @@ p2z_status p2z_run_device(p2z_context *ctx, const p2z_config *cfg, const void *d
   base.nlayer = pl.nlayer;
   base.kfact = pl.kfact;
   base.status = ctx->d_status;
-  const int schedule = resolve_schedule(ctx, pl, cfg, mask != nullptr);
+  const int schedule = resolve_schedule(ctx, pl, cfg, d_hit_mask != nullptr);
   int launches = 0;
   if ((pl.flags & P2Z_FLAG_CHECK_INPUTS) && pl.nslots > 0) {
     // synchronous: the pass runs only on finite inputs
@@ -847,7 +821,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
     if (r != P2Z_OK) return r;
     pl.padding_mask = d_mask;
   }
-  const int schedule = resolve_schedule(ctx, pl, cfg, d_mask != nullptr);
+  const int schedule = resolve_schedule(ctx, pl, cfg, user_mask);
   // The per-event form is timed as it stands: copies first, then one launch per event.
   const bool per_event = schedule == P2Z_SCHED_PER_EVENT;
   // Only the 2-D updates read just the first 6 of the 9 hit words.

@@ -104,11 +104,6 @@ struct RunArgs {
 // 640-700; 3-D update with the FP64 island, 60 events: 191, 172, 161, 161.  Masks
 // all alike (100 x 9600): 205 stored, 210 sorted.
 constexpr int kSortWindow = 128;
-// Runs that leave the schedule open sort from this many slots an SM on: a launch
-// whose warps are all resident at once lasts as long as its longest track anyway.
-// One B200, 2-D update, us per pass, stored order / sorted: 51,000 tracks 18.6 /
-// 20.8, 102,000 30.7 / 30.8, 152,000 41.0 / 39.2, 406,000 88.1 / 81.6.
-constexpr int64_t kSortMinSlotsPerSm = 768;
 // A warp's counts of one group of 32 slots, a byte a key (0..32), cleared by words.
 union KeyCounts {
   uint32_t word[9];

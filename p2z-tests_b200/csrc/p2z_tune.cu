@@ -13,14 +13,14 @@
 
 #include "p2z.h"
 #include "p2z_kernels.cuh"
+#include "p2z_shape.h"
 
 namespace p2z {
 void set_context_free_error(const char *msg);
 int context_device(const p2z_context *ctx);
 cudaStream_t context_stream(const p2z_context *ctx);
 p2z_status context_fail(p2z_context *ctx, p2z_status st, const char *msg);
-p2z_status record_tuned(p2z_context *ctx, const p2z_config *cfg, bool masked, int block, int schedule, int tpt,
-                        bool sort);
+p2z_status record_tuned(p2z_context *ctx, const p2z_config *cfg, bool caller_mask, const Shape &shape);
 }  // namespace p2z
 
 using namespace p2z;
@@ -303,8 +303,8 @@ p2z_status p2z_autotune(p2z_context *ctx, const p2z_config *cfg, const void *d_t
       c.block_threads = 0;
       c.threads_per_track = 0;
       c.flags = cfg->flags;
-      r = record_tuned(ctx, &c, masked, local.block_threads, local.schedule, local.threads_per_track,
-                       (local.flags & P2Z_FLAG_SORT_WINDOWS) != 0);
+      r = record_tuned(ctx, &c, masked, {local.block_threads, local.schedule, local.threads_per_track,
+                                         (local.flags & P2Z_FLAG_SORT_WINDOWS) != 0});
       if (r != P2Z_OK) return r;
       if (top.ms < 0 || local.ms < top.ms) top = local;
     }
