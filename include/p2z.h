@@ -394,7 +394,7 @@ p2z_status p2z_relayout_device(p2z_context *ctx, const p2z_config *from, const p
  * order; p2z_unpack_tracks_device writes a packed output back in the caller's
  * order.  No mask: every track has every layer and the order is unchanged.
  * The copies must not alias the inputs.  Pack: synchronous (its scratch, 152
- * bytes an event and 136 per 512 slots, is the context's reusable device
+ * bytes an event and 137 per 512 slots, is the context's reusable device
  * buffer); unpack: enqueued on `stream` (NULL = the context's).
  * No counterpart in the reference. */
 p2z_status p2z_pack_by_hits_device(p2z_context *ctx, const p2z_config *cfg, const void *d_trk_in,

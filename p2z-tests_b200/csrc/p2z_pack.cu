@@ -103,38 +103,96 @@ __global__ void __launch_bounds__(kWindow) k_pack_count(Events ev, const uint32_
     for (int c = 0; c < kClasses; ++c) rows[((int64_t)e + blockIdx.x) * kClasses + c] = count[part][c];
 }
 
-// One warp per event: its rows' counts become the offsets, from the event's
-// first slot on, of the row's first slot of each class.
-__global__ void __launch_bounds__(128) k_pack_offsets(Events ev, uint32_t *__restrict__ rows) {
-  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// An event's rows' counts become the offsets, from the event's first slot on, of
+// the row's first slot of each class.  Lane l of a warp takes class l, lanes 0 and
+// 1 classes 32 and 33 as well.  The sums over rows [r0, r1):
+struct ClassSums {
+  uint32_t a, b;
+};
+constexpr int kRowsAhead = 8;  // loads in flight; the walk is otherwise a load's latency a row
+__device__ __forceinline__ ClassSums sum_rows(const uint32_t *rows, int64_t r0, int64_t r1) {
   const int lane = threadIdx.x & 31;
-  if (e >= ev.n || ev.beg[e + 1] == ev.beg[e]) return;
-  const int64_t r0 = e + ev.beg[e] / kWindow, r1 = e + (ev.beg[e + 1] - 1) / kWindow;
-  const bool two = lane < kClasses - 32;  // lanes 0 and 1 take classes 32 and 33 as well
-  uint32_t a = 0u, b = 0u;
-#pragma unroll 4
-  for (int64_t r = r0; r <= r1; ++r) {
-    a += rows[r * kClasses + lane];
-    if (two) b += rows[r * kClasses + 32 + lane];
+  const bool two = lane < kClasses - 32;
+  ClassSums s = {0u, 0u};
+#pragma unroll 8
+  for (int64_t r = r0; r < r1; ++r) {
+    s.a += rows[r * kClasses + lane];
+    if (two) s.b += rows[r * kClasses + 32 + lane];
   }
-  uint32_t at = a;
+  return s;
+}
+// The first offset of each class in an event with these sums.
+__device__ __forceinline__ ClassSums first_offsets(ClassSums s) {
+  const int lane = threadIdx.x & 31;
+  uint32_t at = s.a;
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t u = __shfl_up_sync(0xffffffffu, at, o);
     if (lane >= o) at += u;
   }
-  const uint32_t real32 = __shfl_sync(0xffffffffu, at, 31), b0 = __shfl_sync(0xffffffffu, b, 0);
-  at -= a;
-  uint32_t bt = real32 + (lane ? b0 : 0u);
-  for (int64_t r = r0; r <= r1; ++r) {
-    const uint32_t ra = rows[r * kClasses + lane];
-    rows[r * kClasses + lane] = at;
-    at += ra;
-    if (two) {
-      const uint32_t rb = rows[r * kClasses + 32 + lane];
-      rows[r * kClasses + 32 + lane] = bt;
-      bt += rb;
+  const uint32_t real32 = __shfl_sync(0xffffffffu, at, 31), b0 = __shfl_sync(0xffffffffu, s.b, 0);
+  return {at - s.a, real32 + (lane ? b0 : 0u)};
+}
+// Rows [r0, r1) from counts to offsets, the first row's from `at` on.
+__device__ __forceinline__ void place_rows(uint32_t *rows, int64_t r0, int64_t r1, ClassSums at) {
+  const int lane = threadIdx.x & 31;
+  const bool two = lane < kClasses - 32;
+  for (int64_t r = r0; r < r1; r += kRowsAhead) {
+    uint32_t a[kRowsAhead], b[kRowsAhead];
+#pragma unroll
+    for (int j = 0; j < kRowsAhead; ++j) {
+      a[j] = r + j < r1 ? rows[(r + j) * kClasses + lane] : 0u;
+      b[j] = r + j < r1 && two ? rows[(r + j) * kClasses + 32 + lane] : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kRowsAhead; ++j) {
+      if (r + j < r1) {
+        rows[(r + j) * kClasses + lane] = at.a;
+        if (two) rows[(r + j) * kClasses + 32 + lane] = at.b;
+      }
+      at.a += a[j];
+      at.b += b[j];
     }
   }
+}
+__device__ __forceinline__ void event_rows(const Events &ev, int64_t e, int64_t *r0, int64_t *r1) {
+  *r0 = e + ev.beg[e] / kWindow;
+  *r1 = ev.beg[e + 1] == ev.beg[e] ? *r0 : e + (ev.beg[e + 1] - 1) / kWindow + 1;
+}
+
+// Events of at most kWarpRows rows: one warp each.  The others: one CTA each, whose
+// warps share the rows.  (With one warp for every event, one event of a million
+// tracks and one layer took 444 us to pack, now 132, and of 10 million 4211, now 922; with 20
+// layers, a million, 711 and 398.)
+constexpr int64_t kWarpRows = 32;
+__global__ void __launch_bounds__(128) k_pack_offsets(Events ev, uint32_t *__restrict__ rows) {
+  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (e >= ev.n) return;
+  int64_t r0, r1;
+  event_rows(ev, e, &r0, &r1);
+  if (r1 - r0 > kWarpRows) return;
+  place_rows(rows, r0, r1, first_offsets(sum_rows(rows, r0, r1)));
+}
+__global__ void __launch_bounds__(1024) k_pack_offsets_wide(Events ev, const int64_t *__restrict__ events,
+                                                            uint32_t *__restrict__ rows) {
+  __shared__ ClassSums sums[32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t r0, r1;
+  event_rows(ev, events[blockIdx.x], &r0, &r1);
+  const int64_t per = (r1 - r0 + 31) / 32, w0 = min(r1, r0 + warp * per), w1 = min(r1, w0 + per);
+  sums[warp][lane] = sum_rows(rows, w0, w1);
+  __syncthreads();
+  ClassSums all = {0u, 0u}, before = {0u, 0u};
+  for (int w = 0; w < 32; ++w) {
+    const ClassSums s = sums[w][lane];
+    all.a += s.a;
+    all.b += s.b;
+    if (w < warp) {
+      before.a += s.a;
+      before.b += s.b;
+    }
+  }
+  const ClassSums first = first_offsets(all);
+  place_rows(rows, w0, w1, {first.a + before.a, first.b + before.b});
 }
 
 // Sorts kWindow keys, ascending, a key a thread (bitonic: partners in the same
@@ -323,14 +381,18 @@ __global__ void __launch_bounds__(256) k_unpack_direct(const int64_t *__restrict
 
 bool aligned16(const void *a, const void *b) { return (((uintptr_t)a | (uintptr_t)b) & 15u) == 0; }
 
-// Event tables of a config: per-event real tracks and first slots (nevts + 1).
-void event_tables(const p2z_config *c, std::vector<int64_t> &counts, std::vector<int64_t> &beg) {
+// Event tables of a config: per-event real tracks and first slots (nevts + 1), and the
+// events of more than kWarpRows rows.
+void event_tables(const p2z_config *c, std::vector<int64_t> &counts, std::vector<int64_t> &beg,
+                  std::vector<int64_t> &wide) {
   const int64_t ne = c->nevts;
   counts.assign((size_t)ne, 0);
   beg.assign((size_t)ne + 1, 0);
   for (int64_t e = 0; e < ne; ++e) {
     counts[e] = c->event_ntrks ? c->event_ntrks[e] : c->ntrks;
     beg[e + 1] = beg[e] + (counts[e] + c->bsize - 1) / c->bsize * c->bsize;
+    if (counts[e] > (kWarpRows - 1) * kWindow && (beg[e + 1] - 1) / kWindow - beg[e] / kWindow >= kWarpRows)
+      wide.push_back(e);
   }
 }
 
@@ -367,21 +429,24 @@ p2z_status p2z_pack_by_hits_device(p2z_context *ctx, const p2z_config *cfg, cons
     return context_fail(ctx, P2Z_BAD_ARG, "the packed copy must not alias the input");
   PACK_CUDA(ctx, cudaSetDevice(context_device(ctx)));
   cudaStream_t st = stream ? (cudaStream_t)stream : context_stream(ctx);
-  std::vector<int64_t> counts, beg;
-  event_tables(cfg, counts, beg);
+  std::vector<int64_t> counts, beg, wide;
+  event_tables(cfg, counts, beg, wide);
   const int ne = (int)cfg->nevts;
   const int64_t nwin = (ns + kWindow - 1) / kWindow;
   if (nwin > 0x7fffffff) return context_fail(ctx, P2Z_BAD_ARG, "too many slots");
   // scratch, from the context's reusable device buffer (parts 256-byte aligned): event tables and
   // the rows of counts (one per event and window)
-  const size_t b_tab = up256(sizeof(int64_t) * (2 * (size_t)ne + 1));
+  const size_t nwide = wide.size();
+  const size_t b_tab = up256(sizeof(int64_t) * (2 * (size_t)ne + 1 + nwide));
   char *scr = static_cast<char *>(
       context_scratch(ctx, b_tab + up256(sizeof(uint32_t) * kClasses * ((size_t)ne + (size_t)nwin))));
   if (!scr) return context_fail(ctx, P2Z_OOM, "no device memory for the packing scratch");
-  int64_t *d_counts = (int64_t *)scr, *d_beg = d_counts + ne;
+  int64_t *d_counts = (int64_t *)scr, *d_beg = d_counts + ne, *d_wide = d_beg + ne + 1;
   uint32_t *rows = (uint32_t *)(scr + b_tab);
   PACK_CUDA(ctx, cudaMemcpyAsync(d_counts, counts.data(), sizeof(int64_t) * ne, cudaMemcpyHostToDevice, st));
   PACK_CUDA(ctx, cudaMemcpyAsync(d_beg, beg.data(), sizeof(int64_t) * (ne + 1), cudaMemcpyHostToDevice, st));
+  if (nwide)
+    PACK_CUDA(ctx, cudaMemcpyAsync(d_wide, wide.data(), sizeof(int64_t) * nwide, cudaMemcpyHostToDevice, st));
   const Events ev{d_beg, d_counts, ne};
   const int nl = cfg->nlayer;
   const uint32_t all = nl >= 32 ? 0xffffffffu : ((1u << nl) - 1u);
@@ -389,6 +454,10 @@ p2z_status p2z_pack_by_hits_device(p2z_context *ctx, const p2z_config *cfg, cons
   PACK_CUDA(ctx, cudaGetLastError());
   k_pack_offsets<<<(unsigned)(((int64_t)ne * 32 + 127) / 128), 128, 0, st>>>(ev, rows);
   PACK_CUDA(ctx, cudaGetLastError());
+  if (nwide) {
+    k_pack_offsets_wide<<<(unsigned)nwide, 1024, 0, st>>>(ev, d_wide, rows);
+    PACK_CUDA(ctx, cudaGetLastError());
+  }
   // small samples: a window's layers are shared out until the GPU is full
   const int shares = (int)std::max<int64_t>(1, std::min<int64_t>(nl, kFillWindows / nwin));
   const int per = (nl + shares - 1) / shares;
