@@ -118,8 +118,8 @@ typedef enum p2z_update_kind {
 } p2z_update_kind;
 
 /* How the work is laid onto the GPU.
- *  AUTO        FLAT; with a caller's hit mask and enough slots to fill the GPU more than once, FLAT
- *              with P2Z_FLAG_SORT_WINDOWS.
+ *  AUTO        FLAT; with a caller's hit mask, launches of enough slots to fill the GPU more than
+ *              once sort their windows (P2Z_FLAG_SORT_WINDOWS), the 2-D update in batches of 8 apart.
  *  FLAT        one launch over every track slot of every event.
  *  PER_EVENT   one launch per event (the reference's launch-per-chunk form,
  *              src/propagate-toz-test_CUDA_v4.cu:970-986, taken down to one event per launch).

@@ -148,6 +148,7 @@ struct Plan {
   int schedule = P2Z_SCHED_FLAT;
   int block = 0;             // 0: kFlatBlock or kQueueBlock, by the schedule
   int tpt = 1;               // threads per track
+  int64_t sort_from = kNeverSort;  // masked launches of this many slots or more sort their windows
   uint32_t flags = 0;
   int64_t nbatches = 0;
   int64_t nslots = 0;
@@ -371,7 +372,7 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   if (s1 <= s0) return P2Z_OK;
   spec.args.l2_prefetch = prefetch_for(s1 - s0);  // (the staged kernel stages its hits itself)
   // masked flat and persistent runs: process each window's slots in order of hit count
-  const bool sort = spec.masked && !padded && (pl.flags & P2Z_FLAG_SORT_WINDOWS) &&
+  const bool sort = spec.masked && !padded && s1 - s0 >= pl.sort_from &&
                     (schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PERSISTENT);
   spec.args.sort = sort ? 1 : 0;
   if (sort && !pl.block) spec.block = kSortedBlock;
@@ -453,12 +454,12 @@ RunKind run_kind(const Plan &pl, bool caller_mask) {
 int resolve_schedule(const p2z_context *ctx, Plan &pl, const p2z_config *cfg, bool caller_mask) {
   const Shape s = choose_shape(ctx->tuned, run_kind(pl, caller_mask),
                                {cfg->block_threads, cfg->schedule, cfg->threads_per_track,
-                                (pl.flags & P2Z_FLAG_SORT_WINDOWS) != 0},
-                               pl.nslots, ctx->num_sms);
+                                (pl.flags & P2Z_FLAG_SORT_WINDOWS) ? 0 : kNeverSort},
+                               ctx->num_sms);
   pl.block = s.block;
   pl.schedule = s.schedule;
   pl.tpt = s.tpt;
-  if (s.sort) pl.flags |= P2Z_FLAG_SORT_WINDOWS;
+  pl.sort_from = s.sort_from;
   return pl.schedule;
 }
 

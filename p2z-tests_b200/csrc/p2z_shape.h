@@ -26,11 +26,14 @@ struct RunKind {
   }
 };
 
+// Shape::sort_from of runs that never sort.  (P2Z_FLAG_SORT_WINDOWS: 0.)
+constexpr int64_t kNeverSort = INT64_MAX;
+
 struct Shape {
-  int block;     // threads per CTA, 0: the schedule's default
-  int schedule;  // p2z_schedule
-  int tpt;       // threads per track, 0: one
-  bool sort;     // P2Z_FLAG_SORT_WINDOWS
+  int block;          // threads per CTA, 0: the schedule's default
+  int schedule;       // p2z_schedule
+  int tpt;            // threads per track, 0: one
+  int64_t sort_from;  // a masked launch of this many slots or more sorts its windows
 };
 
 // p2z_autotune's fastest shape of one kind of run.
@@ -48,29 +51,36 @@ inline void record_shape(std::vector<Tuned> &tuned, const RunKind &kind, const S
   tuned.push_back({kind, shape});
 }
 
-// Runs that leave the schedule open sort from this many slots an SM on: a launch
-// whose warps are all resident at once lasts as long as its longest track anyway.
-// One B200, 2-D update, us per pass, stored order / sorted: 51,000 tracks 18.6 /
-// 20.8, 102,000 30.7 / 30.8, 152,000 41.0 / 39.2, 406,000 88.1 / 81.6.
+// Launches of runs that leave the schedule open sort from this many slots an SM on:
+// one whose warps are all resident at once lasts as long as its longest track anyway.
+// A launch, not a run: p2z_run cuts a run into chunks, the last ones small.
+// One B200, 32 slots a batch, 2-D update, us per pass, stored order / sorted: 64,000
+// slots 18.1 / 19.4, 113,000 27.5 / 26.2, 154,000 38.3 / 36.8, 306,000 68.9 / 61.9,
+// 1,006,000 201.6 / 172.8; the other updates gain more (reference rounding 549.9 /
+// 408.2, 3-D with FP64 421.4 / 319.9), 64 slots a batch and SoA as much, 16 slots less
+// (203.6 / 181.7).  In batches of 8 a sorted warp's loads reach 16 batches, a sector each:
+// the 2-D update loses (113,000 28.9 / 31.0, 306,000 71.1 / 73.8, 1,004,000 207.3 /
+// 208.7) and keeps the stored order, the others still gain (235.2 / 215.2 the least).
 constexpr int64_t kSortMinSlotsPerSm = 768;
 
 // Fills what `s`, the caller's wishes, leaves open (block 0, schedule AUTO -- with
 // the window sorting measured with it --, tpt 0).  A tuned shape whose schedule
 // the caller overrides with STAGED keeps one thread per track.
-inline Shape choose_shape(const std::vector<Tuned> &tuned, const RunKind &kind, Shape s, int64_t nslots, int num_sms) {
+inline Shape choose_shape(const std::vector<Tuned> &tuned, const RunKind &kind, Shape s, int num_sms) {
   for (const Tuned &t : tuned) {
     if (!(t.kind == kind)) continue;
     if (s.block == 0) s.block = t.shape.block;
     if (s.schedule == P2Z_SCHED_AUTO) {
       s.schedule = t.shape.schedule;
-      s.sort = s.sort || t.shape.sort;
+      if (t.shape.sort_from < s.sort_from) s.sort_from = t.shape.sort_from;
     }
     if (s.tpt == 0 && s.schedule != P2Z_SCHED_STAGED) s.tpt = t.shape.tpt;
     break;
   }
   if (s.schedule == P2Z_SCHED_AUTO) {
     s.schedule = P2Z_SCHED_FLAT;
-    s.sort = s.sort || (kind.mask == MASK_CALLER && nslots >= num_sms * kSortMinSlotsPerSm);
+    const bool scattered = kind.upd == P2Z_UPDATE_V2 && kind.B == 8 && !kind.soa;
+    if (kind.mask == MASK_CALLER && !scattered && s.sort_from == kNeverSort) s.sort_from = num_sms * kSortMinSlotsPerSm;
   }
   if (s.tpt == 0) s.tpt = 1;
   return s;

@@ -304,7 +304,7 @@ p2z_status p2z_autotune(p2z_context *ctx, const p2z_config *cfg, const void *d_t
       c.threads_per_track = 0;
       c.flags = cfg->flags;
       r = record_tuned(ctx, &c, masked, {local.block_threads, local.schedule, local.threads_per_track,
-                                         (local.flags & P2Z_FLAG_SORT_WINDOWS) != 0});
+                                         (local.flags & P2Z_FLAG_SORT_WINDOWS) ? 0 : kNeverSort});
       if (r != P2Z_OK) return r;
       if (top.ms < 0 || local.ms < top.ms) top = local;
     }
