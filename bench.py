@@ -288,9 +288,13 @@ SERVE_RATES = (1000, 2000, 5000, 10000, 20000, 50000)
 
 def tune_summary(best, rows, wall_s):
     """Compact report of an autotune sweep: the fastest row overall, per bsize,
-    per layout and per schedule, and the row the reference's layout gets."""
+    per layout and per schedule, and the row the reference's layout gets.  (A
+    persistent row with sorted windows repeats the flat launch it is, and says
+    nothing of the persistent schedule.)"""
+    own = [r for r in rows if not (r["schedule"] == "persistent" and r["sorted_windows"])]
+
     def fastest(pred):
-        sel = [r for r in rows if pred(r)]
+        sel = [r for r in own if pred(r)]
         return min(sel, key=lambda r: r["ms"]) if sel else None
     out = {"configurations": len(rows), "sweep_wall_s": wall_s, "best": best,
            "best_bsize32_aosoa": fastest(lambda r: r["bsize"] == 32 and r["layout"] == "aosoa")}
@@ -305,26 +309,22 @@ def tune_summary(best, rows, wall_s):
 def small_run_latency(p2z, ctx, t, h, o):
     """Host wall time of one synchronous p2z_run call on a lone event of 1024
     or 9600 tracks from page-locked buffers (the first batches of the bench
-    sample), one pass across the link: the default call and the same with
-    P2Z_FLAG_NO_GRAPH, which changes nothing here; mean of 200 calls after 5
-    warm-up calls."""
+    sample), one pass across the link; mean of 200 calls after 5 warm-up
+    calls."""
     out = {}
     for n in (1024, 9600):
         nb = n // 32
-        row = {}
-        for mode, flags in (("default", 0), ("direct", p2z.FLAG_NO_GRAPH)):
-            cfg = p2z.make_config(bsize=32, nevts=1, ntrks=n, nlayer=20, schedule="flat", flags=flags)
-            args = (ctx.h, p2z.C.byref(cfg), t[:nb].ctypes.data, h[:nb].ctypes.data, None, o[:nb].ctypes.data, None)
-            for _ in range(5):
-                p2z.lib.p2z_run(*args)
-            t0 = time.perf_counter()
-            for _ in range(200):
-                rc = p2z.lib.p2z_run(*args)
-            us = (time.perf_counter() - t0) / 200 * 1e6
-            if rc != p2z.OK:
-                raise p2z.P2zError(rc, p2z.lib.p2z_last_error(ctx.h).decode())
-            row[mode + "_us"] = us
-        out[str(n)] = row
+        cfg = p2z.make_config(bsize=32, nevts=1, ntrks=n, nlayer=20, schedule="flat")
+        args = (ctx.h, p2z.C.byref(cfg), t[:nb].ctypes.data, h[:nb].ctypes.data, None, o[:nb].ctypes.data, None)
+        for _ in range(5):
+            p2z.lib.p2z_run(*args)
+        t0 = time.perf_counter()
+        for _ in range(200):
+            rc = p2z.lib.p2z_run(*args)
+        us = (time.perf_counter() - t0) / 200 * 1e6
+        if rc != p2z.OK:
+            raise p2z.P2zError(rc, p2z.lib.p2z_last_error(ctx.h).decode())
+        out[str(n)] = {"default_us": us}
     return {"note": "p2z_run from page-locked buffers, one event, host wall time per synchronous call",
             "tracks": out}
 
@@ -747,7 +747,8 @@ def main():
         e2e = {"value": updates * world / (e2e_ms / 1e3), "unit": "updates/s",
                "h2d_bytes_per_step": int(s.h2d_bytes), "d2h_bytes_per_step": int(s.d2h_bytes),
                "ms_per_step": e2e_ms, "steps": n_e2e,
-               "path": "p2z_run, pinned host buffers, 16 chunks on 2 streams (copy/compute overlap)",
+               "path": "p2z_run, pinned host buffers, chunks of a third of what is left: copies in on one stream, "
+                       "passes and copies back on another",
                "roofline": {"bound": "host link (PCIe)", "link_floor_ms": link_ms, "frac": link_ms / e2e_ms,
                             "ceiling_updates_per_s": updates * world / (link_ms / 1e3),
                             "peaks": {k: live_peaks[k] for k in ("h2d_gbs", "d2h_gbs", "bidir_gbs")},
@@ -782,8 +783,8 @@ def main():
             best, rows = ctx.autotune(ucfg, udt, udh, d_mask=udm, reps=3)
             tune_uneven = tune_summary(best, rows, time.time() - t0)
             for sched in blocks:
-                r = min((r for r in rows if r["bsize"] == 32 and r["layout"] == "aosoa" and r["schedule"] == sched),
-                        key=lambda r: r["ms"])
+                r = min((r for r in rows if r["bsize"] == 32 and r["layout"] == "aosoa" and r["schedule"] == sched
+                         and not r["sorted_windows"]), key=lambda r: r["ms"])
                 blocks[sched] = r["block_threads"]
         def timed(c, t, h, mk, o):
             """updates/s of c on (t, h, mk) -> o, CUDA events on our stream, max over ranks"""
@@ -816,10 +817,11 @@ def main():
             tuned_rate = timed(p2z.make_config(bsize=32, nevts=len(counts), event_ntrks=counts, nlayer=20,
                                                schedule="auto", block_threads=0, threads_per_track=0),
                                udt, udh, udm, udo)
-        # the same batched run with each 128-slot window in order of hit count (in-library sort)
-        csw = cfg_for("persistent")
+        # one flat launch with each 128-slot window in order of hit count (in-kernel sort)
+        csw = cfg_for("flat")
         csw.flags |= p2z.FLAG_SORT_WINDOWS
-        res["persistent_sorted_windows"] = timed(csw, udt, udh, udm, udo)
+        csw.block_threads = 0
+        res["sorted_windows"] = timed(csw, udt, udh, udm, udo)
         # the plain form as the reference's GPU build issues it: launches spread over 10 streams
         c10 = cfg_for("per_event")
         c10.flags |= p2z.FLAG_PER_EVENT_STREAMS
@@ -869,7 +871,7 @@ def main():
                "tracks": int(counts.sum()), "updates_per_step": u_upd,
                "batched_persistent_graph": res["persistent"], "plain_per_event_launch": res["per_event"],
                "plain_per_event_launch_10_streams": res["per_event_10_streams"],
-               "batched_persistent_graph_sorted_windows": res["persistent_sorted_windows"],
+               "batched_flat_sorted_windows": res["sorted_windows"],
                "batched_autotuned": ({"updates_per_s": tuned_rate,
                                       "shape": {k: tune_uneven["best_bsize32_aosoa"][k] for k in
                                                 ("schedule", "block_threads", "threads_per_track", "sorted_windows")}}
@@ -890,7 +892,7 @@ def main():
                    "fp32_frac_reference_form": {
                        k: FLOPS_PER_UPDATE_REFERENCE_FORM * v / 1e12 / fp32_peak_live
                        for k, v in (("stored_order", res["persistent"]),
-                                    ("sorted_windows", res["persistent_sorted_windows"]),
+                                    ("sorted_windows", res["sorted_windows"]),
                                     ("ordered_by_hits", ordered["persistent"]),
                                     ("library_packing", lib_pack["batched_persistent_graph"]))},
                    "note": "present-hit updates; bytes = 24 per present hit + 228 per real track (in, out, mask); "

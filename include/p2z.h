@@ -422,7 +422,8 @@ typedef struct p2z_tune_entry {
  * {32,64,128,256} x threads_per_track {1, and 2 where the update kind and
  * schedule have it} x, for masked runs on the FLAT and PERSISTENT schedules,
  * window sorting {off, P2Z_FLAG_SORT_WINDOWS}, each the mean
- * of `reps` passes (0 -> 3) after one warm-up pass.  The inputs are converted
+ * of `reps` passes (0 -> 3) after one warm-up pass (sorted windows are the same
+ * launch under both schedules: the PERSISTENT rows repeat the FLAT ones').  The inputs are converted
  * to each candidate's bsize and layout with p2z_relayout_device into scratch
  * buffers the call allocates and frees (about twice the input size); the
  * caller's buffers are only read.  Results: the number of configurations

@@ -375,7 +375,10 @@ p2z_status enqueue_pass(p2z_context *ctx, const Plan &pl, const RunArgs &base, i
   const bool sort = spec.masked && !padded && s1 - s0 >= pl.sort_from &&
                     (schedule == P2Z_SCHED_FLAT || schedule == P2Z_SCHED_PERSISTENT);
   spec.args.sort = sort ? 1 : 0;
-  if (sort && !pl.block) spec.block = kSortedBlock;
+  if (sort) {  // one flat launch, whichever schedule asks for it
+    spec.early = pl.early;
+    if (!pl.block) spec.block = kSortedBlock;
+  }
   if (schedule == P2Z_SCHED_FLAT || sort) {
     spec.kind = KIND_FLAT;
     P2Z_CUDA(ctx, dispatch(spec, st));

@@ -103,3 +103,17 @@ def test_chunks_on_both_sides_of_the_limit(p2z, ctx, pinned):
     out = torch.empty(dt.shape, pin_memory=pinned)
     ctx.run(cfg, t, h, out, hit_mask=m)
     assert torch.equal(out.view(torch.int32), want.cpu().view(torch.int32))
+
+
+@pytest.mark.gpu
+def test_autotune_measures_a_sorted_launch_once(p2z, ctx):
+    """Sorted windows are one flat launch under either schedule: both rows of the sweep give one
+    figure, and the fastest row names the flat one."""
+    cfg, dt, dh, dm = _masked(p2z, ctx, 32, 6400)
+    with p2z.Context(0) as c:
+        best, rows = c.autotune(cfg, dt, dh, d_mask=dm, reps=1)
+    key = lambda r: (r["bsize"], r["layout"], r["threads_per_track"], r["block_threads"])  # noqa: E731
+    flat, queue = ({key(r): r["ms"] for r in rows if r["schedule"] == s and r["sorted_windows"]}
+                   for s in ("flat", "persistent"))
+    assert len(flat) == 4 * 2 * 2 * 4 and flat == queue
+    assert not (best["schedule"] == "persistent" and best["sorted_windows"])
