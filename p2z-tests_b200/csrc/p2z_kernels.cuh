@@ -61,8 +61,9 @@ struct Types {
   // Register budget: kernels allow up to 256 threads per CTA and ask ptxas
   // for MIN_CTAS such CTAs per SM.  For the 2-D FP32 kinds, 3 caps them at 80
   // registers (24 resident warps per SM), which measured faster than the 88
-  // ptxas picks unconstrained (the reference-rounding kind spills 36 bytes at 80
-  // and is 1.5% faster than with its own 96 all the same).  For the 3x3 update with its FP64 island, 2
+  // ptxas picks unconstrained (the reference-rounding flat kernels spill 24-56 bytes at
+  // 80, the masked SoA one none, and are 1.5% faster than with their own 96 all the
+  // same; its staged kernel is exempt).  For the 3x3 update with its FP64 island, 2
   // caps it at 128 (16 warps instead of the 12 that 157-164 registers allow;
   // with the Joseph form evaluated a row at a time the cap spills 4 bytes):
   // 4.44 against 4.51 ms on the headline sample, 4.32 against 5.63 ms on the
@@ -591,8 +592,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
                : "memory");
 }
 
+// (The reference rounding keeps the registers ptxas gives it, 90 and masked 128: at 80
+// the masked kernel spills, and 120,000 masked tracks took 144-153 us instead of 106.)
 template <int UPD, int SC, bool MASKED>
-__global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_staged(RunArgs a) {
+__global__ void __launch_bounds__(256, UPD == UPDK_V2_REF ? 1 : Types<UPD>::MIN_CTAS) k_staged(RunArgs a) {
   constexpr int B = 32;
   constexpr int NH = Types<UPD>::NH;
   using SM = StagedSmem<UPD>;
