@@ -284,12 +284,16 @@ __device__ __forceinline__ void copy_async_4(uint32_t dst, const float *src) {
 // The masked 3-D kernels' ring: a lane's own words of its next present layers.
 // Lanes at different layers, and sorted windows more so, touch many sectors a
 // load; at 9 words a layer and 16 warps an SM the next layer in registers did not
-// cover that (one B200, 60 masked events, sorted, us per pass: registers 147, a
-// ring of 3 or 4 stages 139).  The 2-D kernels' 24 warps do without (500 masked
-// events, under the power cap: 569 with registers, 577 with the ring).
+// cover that (one B200, 60 masked events, FP64 island, sorted, us per pass: registers
+// 147, a ring of 3 or 4 stages 139).  The 2-D kernels' 24 warps do without (500 masked
+// events, under the power cap: 569 with registers, 577 with the ring), and so does
+// the FP32 3-D update's queue kernel (300,000 masked tracks 105 and 109, SoA without a
+// mask 60,000 32.5 and 34.5; sorted flat launches 85 and 81).
 constexpr int kMaskedRing = 3;
-template <int UPD, bool MASKED, int TPT>
-constexpr bool uses_ring() { return MASKED && TPT == 1 && Types<UPD>::NH == 9; }
+template <int UPD, bool MASKED, int TPT, bool QUEUE>
+constexpr bool uses_ring() {
+  return MASKED && TPT == 1 && (UPD == UPDK_3X3_F64 || (UPD == UPDK_3X3_COMP && !QUEUE));
+}
 template <int UPD>
 constexpr int masked_ring_words() { return kMaskedRing * Types<UPD>::NH * 32; }  // a warp
 
@@ -306,8 +310,8 @@ __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.
 
 // Process one track slot: load, run every present layer, store.  TPT = 2: both
 // lanes of the pair load the track and its hits, and lane 0 stores the result.
-template <int B, int UPD, int SC, bool MASKED, int TPT = 1>
-__device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot, float *ring = nullptr) {
+template <int B, int UPD, int SC, bool MASKED, int TPT, bool QUEUE>
+__device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot, float *ring) {
   using T = typename Types<UPD>::T;
   using A = typename Types<UPD>::A;
   constexpr int NH = Types<UPD>::NH;
@@ -324,7 +328,7 @@ __device__ __forceinline__ void process_slot(const RunArgs &a, int64_t slot, flo
   const uint32_t all = (a.nlayer >= 32) ? 0xffffffffu : ((1u << a.nlayer) - 1u);
   uint32_t m = MASKED ? (__ldg(a.mask + slot) & all) : all;
   // the ring's copies start before the track's words are needed
-  constexpr bool RING = uses_ring<UPD, MASKED, TPT>();
+  constexpr bool RING = uses_ring<UPD, MASKED, TPT, QUEUE>();
   uint32_t todo = m, ring_dst = 0u;
   const float *ring_src = nullptr;
   int fill = 0;
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_flat(RunArgs a) {
   }
   if (slot >= a.slot_end) return;  // (both lanes of a pair together)
   extern __shared__ __align__(16) float hit_ring[];
-  process_slot<B, UPD, SC, MASKED, TPT>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
+  process_slot<B, UPD, SC, MASKED, TPT, false>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
 }
 
 // Persistent launch: grid = resident CTAs; each warp repeatedly takes the next
@@ -523,7 +527,7 @@ __global__ void __launch_bounds__(256, Types<UPD>::MIN_CTAS) k_persistent(RunArg
     if (item >= nitems) break;
     const int64_t slot = a.slot_begin + (int64_t)item * kPer + lane / TPT;
     if (slot < a.slot_end)
-      process_slot<B, UPD, SC, MASKED, TPT>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
+      process_slot<B, UPD, SC, MASKED, TPT, true>(a, slot, hit_ring + (threadIdx.x >> 5) * masked_ring_words<UPD>());
   }
 }
 
@@ -871,7 +875,8 @@ struct Dispatch {
   }
   // dynamic shared memory of a launch
   static size_t smem_bytes(const LaunchSpec &s) {
-    if (s.masked && uses_ring<UPD, true, 1>() && s.kind != KIND_STAGED)
+    if (s.masked && ((s.kind == KIND_FLAT && uses_ring<UPD, true, 1, false>()) ||
+                     (s.kind == KIND_PERSISTENT && uses_ring<UPD, true, 1, true>())))
       return (size_t)(s.block / 32) * masked_ring_words<UPD>() * sizeof(float);
     return s.kind == KIND_STAGED ? (size_t)(s.block / 32) * StagedSmem<UPD>::kWarpBytes : 0;
   }
