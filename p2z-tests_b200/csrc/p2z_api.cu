@@ -818,8 +818,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
     ctx->mask_key.clear();
     d_mask = (const uint32_t *)ctx->mask.p;
   }
-  // sc carries the host->device copies; sp the passes and the copies back
-  cudaStream_t sc = ctx->copy[0], sp = ctx->copy[1];
+  cudaStream_t sp = ctx->copy[1];
   if (!user_mask && pl.uneven) {
     r = internal_mask(ctx, pl, sp, &d_mask);
     if (r != P2Z_OK) return r;
@@ -866,6 +865,13 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
     first.push_back(left - take < least || first.size() == kRunMaxChunks ? pl.nbatches : first.back() + take);
   }
   const int nchunk = (int)first.size() - 1;
+  // sc carries the host->device copies; sp the passes and the copies back.  One chunk
+  // of pageable memory, whose copies hold up the host anyway, stays on one stream (1024
+  // masked tracks, wall us a call: 123-126, with two streams and their events 130; from
+  // page-locked memory two streams are the faster, 256 tracks 73 and 80).
+  HostRange locked;
+  const bool two_streams = nchunk > 1 || direct || page_locked_range((uintptr_t)trk_in, &locked);
+  cudaStream_t sc = two_streams ? ctx->copy[0] : sp;
   int launches = 0;
   int64_t h2d = 0, d2h = 0;
   P2Z_CUDA(ctx, cudaEventRecord(ctx->ev0, sc));
@@ -876,7 +882,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
   for (int it = 0; it < pl.niter; ++it) {
     for (int c = 0; c < nchunk; ++c) {
       const int64_t b0 = first[c], b1 = first[c + 1], nbc = b1 - b0;
-      if (it > 0) P2Z_CUDA(ctx, cudaStreamWaitEvent(sc, ctx->passed[c], 0));
+      if (two_streams && it > 0) P2Z_CUDA(ctx, cudaStreamWaitEvent(sc, ctx->passed[c], 0));
       if (direct) {
         h2d += (int64_t)read_bytes;
       } else if (pl.soa) {
@@ -905,8 +911,10 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
                                       nbc * pl.B * 4, cudaMemcpyHostToDevice, sc));
         h2d += nbc * pl.B * 4;
       }
-      P2Z_CUDA(ctx, cudaEventRecord(ctx->arrived[c], sc));
-      P2Z_CUDA(ctx, cudaStreamWaitEvent(sp, ctx->arrived[c], 0));
+      if (two_streams) {
+        P2Z_CUDA(ctx, cudaEventRecord(ctx->arrived[c], sc));
+        P2Z_CUDA(ctx, cudaStreamWaitEvent(sp, ctx->arrived[c], 0));
+      }
       if (check) {
         r = enqueue_check(ctx, pl, base, b0 * pl.B, b1 * pl.B, sp);
         if (r != P2Z_OK) return r;
@@ -925,7 +933,7 @@ p2z_status p2z_run(p2z_context *ctx, const p2z_config *cfg, const void *trk_in, 
                                       cudaMemcpyDeviceToHost, sp));
       }
       d2h += nbc * tb;
-      if (it + 1 < pl.niter) P2Z_CUDA(ctx, cudaEventRecord(ctx->passed[c], sp));
+      if (two_streams && it + 1 < pl.niter) P2Z_CUDA(ctx, cudaEventRecord(ctx->passed[c], sp));
     }
   }
   P2Z_CUDA(ctx, cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, sp));
