@@ -37,12 +37,12 @@ constexpr int kRunMaxChunks = 16;  // ln(64)/ln(3/2) + 1 of them at most, and th
 constexpr int kEventStreams = 10;
 // Threads per CTA where neither the caller nor the autotuner says: flat launches
 // take CTAs of one warp, which leave their registers as soon as the warp is done
-// (one B200, us per pass with 32 / 128: 100 x 9600 tracks 188.5 / 194.6, 500 masked
-// events in stored order 606 / 610).  Sorted windows take the window's four warps
+// (one B200, us per pass with 32 / 128 / 256: a million masked tracks in stored order
+// 201.0 / 202.4 / 208.4, with the 3-D update 421.5 / 423.6 / 435.4; 100 x 9600 tracks
+// without a mask 186.5 / 186.8).  Sorted windows take the window's four warps
 // as one CTA: they read the same sectors of hits, which one SM's L1 then holds for
-// all of them (500 masked events, under the power cap that a longer load meets,
-// 627 / 577, 60 with the 3-D update 143 / 139).  The queue kernels' warps fetch their
-// next work themselves.
+// all of them (500 masked events 613 / 548 / 579, 60 with the 3-D update 141 / 131 /
+// 152).  The queue kernels' warps fetch their next work themselves.
 constexpr int kFlatBlock = 32, kSortedBlock = p2z::kSortWindow, kQueueBlock = 128;
 namespace p2z {
 cudaError_t launch_step(int bsize, float *trk, const float *hits, int64_t nslots, int nlayer, int layer, int what,

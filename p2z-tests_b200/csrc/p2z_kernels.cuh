@@ -101,9 +101,9 @@ struct RunArgs {
 // registers for a longer one.  The window: 5-20 hits a track keep 61% of the
 // lane-steps busy in stored order, 74 / 85 / 92% in windows of 64 / 128 / 256,
 // but a warp's loads then reach 2 / 4 / 8 batches.  One B200, 500 uneven events,
-// 2-D update, us per pass: stored order 606, windows of 64 545, 128 533-570, 256
-// 640-700; 3-D update with the FP64 island, 60 events: 191, 172, 161, 161.  Masks
-// all alike (100 x 9600): 205 stored, 210 sorted.
+// 2-D update, us per pass: stored order 616, windows of 64 542, 128 548, 256
+// 620; 3-D update with the FP64 island, 60 events: 169, 145, 131, 137.  Masks
+// all alike (100 x 9600): 203 stored, 209 sorted.
 constexpr int kSortWindow = 128;
 // A warp's counts of one group of 32 slots, a byte a key (0..32), cleared by words.
 union KeyCounts {
@@ -304,7 +304,8 @@ constexpr int masked_ring_words() { return kMaskedRing * Types<UPD>::NH * 32; } 
 // the next launch let in at the start, 64,000 tracks took 27.1 us where they take
 // 19.1), no later, so that the set-up hides behind the stores.  Without the
 // attribute both do nothing.  One B200, passes queued behind one another, us each,
-// with / without: one event of 1024 tracks 7.9 / 10.2, 64 x 4096 tracks 54.2 / 57.3.
+// with / without: one event of 1024 tracks 7.9 / 10.2, 30,000 tracks 9.7 / 12.4,
+// 300,000 63.2 / 65.6.
 __device__ __forceinline__ void start_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 

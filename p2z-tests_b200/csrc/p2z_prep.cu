@@ -144,8 +144,8 @@ __device__ __forceinline__ bool accepted(int32_t d1, int32_t d2, float *u1, floa
 // log of a normal float in (0, 1) in double, to about 1e-16 relative (the caller
 // rounds it to float): w = 2^e m with m in [1/sqrt 2, sqrt 2), and log m = 2 atanh s
 // = 2 s (1 + s^2/3 + s^4/5 + ...) with s = (m - 1)/(m + 1), |s| <= 0.1716 (the
-// next term, s^22/23, is below 1e-18).  The quotient: the MUFU reciprocal
-// (23 bits) after one Newton step, and one correction of the quotient itself.
+// next term, s^22/23, is below 1e-18).  The quotient by Newton's iteration: one step
+// on the hardware's approximate reciprocal, then the quotient corrected by its residual.
 // (With CUDA's log(double), which covers every double, k_emit took 150 us where it
 // takes 136.)  Its float agrees with the rounded logarithm on 3e7 values of the range.
 __device__ __forceinline__ double log01(float w) {
