@@ -577,6 +577,7 @@ void set_context_free_error(const char *msg) { fail(nullptr, P2Z_OK, "%s", msg);
 // Autotuner hooks: the context's device and stream, its error message, and
 // the record of a measured best launch shape for the runs cfg describes.
 int context_device(const p2z_context *ctx) { return ctx->device; }
+int context_sms(const p2z_context *ctx) { return ctx->num_sms; }
 cudaStream_t context_stream(const p2z_context *ctx) { return ctx->stream; }
 p2z_status context_fail(p2z_context *ctx, p2z_status st, const char *msg) { return fail(ctx, st, "%s", msg); }
 // Device scratch owned by the context, at least `bytes` long (nullptr on failure).

@@ -31,6 +31,7 @@
 namespace p2z {
 void set_context_free_error(const char *msg);
 int context_device(const p2z_context *ctx);
+int context_sms(const p2z_context *ctx);
 cudaStream_t context_stream(const p2z_context *ctx);
 p2z_status context_fail(p2z_context *ctx, p2z_status st, const char *msg);
 void *context_scratch(p2z_context *ctx, size_t bytes);
@@ -56,7 +57,8 @@ size_t up256(size_t n) { return (n + 255) / 256 * 256; }
 constexpr int kWindow = 512;   // slots, one a thread
 constexpr int kClasses = 34;   // 32 - hit count of a real track (0: all of 32 layers), 33 padding
 constexpr int kMaxParts = 64;  // events a window can meet (bsize 8)
-constexpr int64_t kFillWindows = 148 * 4;  // CTAs that fill the GPU
+constexpr int kFillPerSm = 4;    // CTAs an SM that fill the GPU
+constexpr int kUnpackPerSm = 6;  // windows an SM from which unpacking goes through shared memory
 
 // The events' tables on the device: slots from beg[e] on, count[e] real tracks.
 struct Events {
@@ -459,7 +461,7 @@ p2z_status p2z_pack_by_hits_device(p2z_context *ctx, const p2z_config *cfg, cons
     PACK_CUDA(ctx, cudaGetLastError());
   }
   // small samples: a window's layers are shared out until the GPU is full
-  const int shares = (int)std::max<int64_t>(1, std::min<int64_t>(nl, kFillWindows / nwin));
+  const int shares = (int)std::max<int64_t>(1, std::min<int64_t>(nl, (int64_t)kFillPerSm * context_sms(ctx) / nwin));
   const int per = (nl + shares - 1) / shares;
   auto *f = cfg->bsize == 8 ? k_pack_move<8> : cfg->bsize == 16 ? k_pack_move<16> : cfg->bsize == 32 ? k_pack_move<32>
                                                                                                      : k_pack_move<64>;
@@ -489,10 +491,10 @@ p2z_status p2z_unpack_tracks_device(p2z_context *ctx, const p2z_config *cfg, con
   if (nwin > 0x7fffffff) return context_fail(ctx, P2Z_BAD_ARG, "too many slots");
   auto *f = cfg->bsize == 8 ? k_unpack<8> : cfg->bsize == 16 ? k_unpack<16> : cfg->bsize == 32 ? k_unpack<32>
                                                                                                : k_unpack<64>;
-  // through the inverse permutation (d_perm's second half); below 6 windows an SM the window's
-  // sort costs more than the scattered reads (one B200, us: 92,000 slots 10.7 with it, 8.8
+  // through the inverse permutation (d_perm's second half); below kUnpackPerSm windows an SM the
+  // window's sort costs more than the scattered reads (one B200, us: 92,000 slots 10.7 with it, 8.8
   // without, 520,000 39.0 and 41.8, 3.2M 156 and 240)
-  if (nwin < 6 * 148)
+  if (nwin < (int64_t)kUnpackPerSm * context_sms(ctx))
     k_unpack_direct<<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(d_perm + ns, ns, cfg->bsize,
                                                                   (const uint32_t *)d_trk_packed, (uint32_t *)d_trk_out);
   else
