@@ -174,9 +174,11 @@ typedef enum p2z_layout {
                                        PERSISTENT too), so a warp's 32
                                        tracks take similar numbers of steps.  Per-track results are
                                        the same.  On uneven samples lane utilisation
-                                       rises from 60% to 85% and the pass is 6-16% faster;
-                                       a warp's loads then reach 4 batches; on even work (every
-                                       mask alike) it costs 2.5%.  p2z_autotune measures both for
+                                       rises from 60% to 85% and a pass of 120,000 slots or
+                                       more is 4-26% faster, by update, layout and batch width;
+                                       a warp's loads then reach 4 batches of 32 (16 of 8, where
+                                       the 2-D update loses 1-10%); on even work (every
+                                       mask alike) it costs 3%.  p2z_autotune measures both for
                                        masked runs, and runs with schedule AUTO then sort when that
                                        measured faster.  Packing an event's tracks in order of hit
                                        count (p2z_pack_by_hits_device, or when the arrays are built)
